@@ -1123,10 +1123,12 @@ def main():
     stats = torch.zeros(8, dtype=torch.int64, device=dev)
     stream = torch.cuda.current_stream()
 
+    # the counting pass names the replay walk, the one the plain call runs
     def ao_frame(with_stats=False, tris_buf=None, out=None):
         mb.render_ao(pixels if out is None else out, (w, h), cam, builder.m_rootNode, builder.m_internals,
                      d_tris if tris_buf is None else tris_buf, 1, wl["ns"], wl["radius"], 12345,
-                     stats=stats if with_stats else None)
+                     stats=stats if with_stats else None,
+                     traversal=mb.TRAVERSAL_REPLAY if with_stats else mb.TRAVERSAL_STACKFREE)
 
     # counting pass: rays, node visits and triangle tests of one frame (the
     # traversal is deterministic, so every timed frame does the same work)

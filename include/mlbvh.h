@@ -54,7 +54,9 @@ enum {
 };
 enum { MLBVH_RAY_QUERY_CLOSEST = 0, MLBVH_RAY_QUERY_ANY = 1 }; /* RAY_QUERY, minimum_lbvh.h:975 */
 enum {
-    MLBVH_TRAVERSAL_STACKFREE = 0,   /* intersect_stackfree,   minimum_lbvh.h:981  */
+    /* intersect_stackfree, minimum_lbvh.h:981: its Hit records, through the
+     * replay walk's kernels (below) */
+    MLBVH_TRAVERSAL_STACKFREE = 0,
     MLBVH_TRAVERSAL_ESCAPE_LINK = 1, /* intersect_escape_link, minimum_lbvh.h:1063 */
     MLBVH_TRAVERSAL_STACKFULL = 2,   /* intersect_stackfull,   minimum_lbvh.h:912  */
     /* intersect_stackfree's Hit records (bit for bit, ties included) from a walk
@@ -395,9 +397,9 @@ MLBVH_API mlbvh_status mlbvh_render_ao(uint32_t* dPixels, uint32_t* dOccluded, i
                              unsigned long long* dStats, void* dScratch, size_t scratchBytes, void* stream);
 
 /* mlbvh_render_ao with the walk of its rays chosen: MLBVH_TRAVERSAL_STACKFREE
- * (what mlbvh_render_ao runs) or MLBVH_TRAVERSAL_REPLAY (the same occlusion
- * counts and pixels from fewer node loads; primary rays too). With REPLAY,
- * dLeafTriangles (may be NULL) is the tree's triangles in leaf order from
+ * (what mlbvh_render_ao takes) or MLBVH_TRAVERSAL_REPLAY. Both give the same
+ * occlusion counts and pixels, and without dStats both run the replay walk's
+ * kernels. With REPLAY, dLeafTriangles (may be NULL) is the tree's triangles in leaf order from
  * mlbvh_leaf_triangles: 16-byte aligned records read with three vector loads
  * instead of nine scalar ones, same results. No reference counterpart. With
  * dStats, node visits are those of the chosen walk. */
@@ -487,10 +489,10 @@ MLBVH_API mlbvh_status mlbvh_render_pt(float* dAccumulators, int width, int heig
                              const mlbvh_triangle* dTriangles, const mlbvh_triangle_attrib* dAttribs,
                              int useSobol, int maxSPP, int maxDepth, void* stream);
 /* mlbvh_render_pt with the walk of its closest-hit rays chosen:
- * MLBVH_TRAVERSAL_STACKFREE (what mlbvh_render_pt runs) or
- * MLBVH_TRAVERSAL_REPLAY (the same Hit records, so the same accumulators,
- * from fewer node loads; dLeafTriangles from mlbvh_leaf_triangles may be
- * NULL). No reference counterpart. */
+ * MLBVH_TRAVERSAL_STACKFREE (what mlbvh_render_pt takes) or
+ * MLBVH_TRAVERSAL_REPLAY, which reads dLeafTriangles (from
+ * mlbvh_leaf_triangles; may be NULL). Both run the replay walk: the same Hit
+ * records, so the same accumulators. No reference counterpart. */
 MLBVH_API mlbvh_status mlbvh_render_pt_ex(float* dAccumulators, int width, int height,
                                           const mlbvh_ray_generator* camera, const mlbvh_node_index* dRootNode,
                                           const mlbvh_internal_node* dInternals, const mlbvh_triangle* dTriangles,
