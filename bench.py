@@ -301,7 +301,7 @@ def bench_batched(args, dev, stream, barrier, max_over_ranks, world, n_meshes=10
         ev[i][1].record(stream)
     for i in range(steps):
         bev[i][0].record(stream)
-        mb.profile_events(*kev[i])  # around k_batch_build, the climb
+        mb.profile_events(*kev[i])  # around the tree kernels
         bb.build(params)
         bev[i][1].record(stream)
         tev[i][0].record(stream)
@@ -972,7 +972,7 @@ def profile_case(name, dev):
     <kernel>), with the inputs larger than L2 and a few GB on the device at
     most. No timing; prints what ran.
       build                   4M-triangle soup: the build chain (k_scene_bounds,
-                              k_keys, 4 x sort::k_onesweep, k_build)
+                              k_keys, 4 x sort::k_onesweep, k_tree_tiles, k_tree_groups, k_tree_cross)
       ao_rays                 4M soup, one 1920x1080 AO frame (64 rays of
                               radius 0.1): k_ao_primary, k_ao_rays, k_ao_finish
       ao_rays_wide(_quantised) the same frame over the 4-wide tree (its
@@ -1255,7 +1255,7 @@ def main():
             if flush is not None:
                 flush.zero_()
             bev[i][0].record(stream)
-            mb.profile_events(*cbev[i])  # around the agglomerative climb (k_build)
+            mb.profile_events(*cbev[i])  # around the tree kernels (k_tree_tiles, _groups, _cross)
             builder.build(d_tris, n, 0, sorter)
             bev[i][1].record(stream)
         torch.cuda.synchronize()
@@ -1381,9 +1381,9 @@ def main():
                    "ao_rays": ao_rays, "parallelism": "replicas" if world > 1 else "single GPU",
                    "l2": "inputs larger than L2 (nodes + triangles 419 MB)" if wl["scene"] == "soup"
                    else "L2 flushed (256 MB write) between timed frames"},
-        "gpu_launches": args.steps * (3 + 3 + 3 + 3 + 3 + 2 + 1 + 7 + 10 + 12),  # AO, replay, quantised, wide, wide
+        "gpu_launches": args.steps * (3 + 3 + 3 + 3 + 3 + 2 + 1 + 9 + 12 + 14),  # AO, replay, quantised, wide, wide
         # quantised AO, wide prep, quantisation,
-        # build, e2e steps, chosen-form e2e steps (7 build + 2 prep + 3 AO)
+        # build, e2e steps, chosen-form e2e steps (9 build + 2 prep + 3 AO)
         "clocks": clocks,
     }
     # roofline of the dominant kernel (k_ao_rays): algorithmic bytes of its rays

@@ -20,7 +20,7 @@
 //                     histograms per mesh, reset of the hand-off words
 //   k_onesweep x P    segmented Onesweep passes (onesweep.cuh), one segment
 //                     per mesh; P = 4 (8-bit digits) or 3 (11-bit digits)
-//   k_batch_build     one thread per sorted leaf: the tile climb of mlbvh_build
+//   k_tree_tiles, k_tree_cross   the trees, as mlbvh_build (tree.cuh)
 //
 // Traversal: k_batch_trace is persistent (one grid of resident CTAs). A warp
 // takes `queueChunk` consecutive rays per atomic on the queue counter and
@@ -37,6 +37,7 @@
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
+#include "tree.cuh"
 
 namespace mlbvh {
 
@@ -45,7 +46,6 @@ namespace {
 constexpr int kPlanThreads = 1024;
 constexpr int kTileThreads = 256;  // bounds / keys kernels: one CTA per sort tile
 constexpr int kStageTris = 256;    // triangles staged in shared memory per step
-constexpr int kBuildThreads = (int)kTileLeaves;  // build: one CTA per tile of the climb
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
 constexpr uint32_t kMaxMeshes = 1u << 20;
 // error word bits: 1 a bounded wait gave up (set by sort::k_onesweep), 2 bad offsets
@@ -54,6 +54,7 @@ constexpr uint32_t kErrOffsets = 2u;
 // header words
 constexpr int kHdrError = 0;
 constexpr int kHdrTickets = 1;  // 4 tile tickets, one per sort pass
+constexpr int kHdrTreeFlags = 5;  // tree::Scratch::flags; the record count follows
 constexpr int kHdrQueue = 8;    // traversal queue counter
 
 struct BatchLayout {
@@ -62,8 +63,10 @@ struct BatchLayout {
     size_t bounds;     // nMeshes x 6 u32 (order-preserving integer form)
     size_t histogram;  // nMeshes x passes x bins u32
     size_t lookback;   // passes x maxTiles x bins u32
+    size_t treeCounts; // tree::count_bytes(n)
     size_t zeroEnd;    // [histogram, zeroEnd) is zeroed by k_batch_bounds
     size_t keysA, keysB, valsA, valsB, handoff;
+    size_t summary;  // tree::summary_bytes(n)
     size_t total;
     uint32_t maxTiles;
 };
@@ -86,6 +89,8 @@ BatchLayout batch_layout(uint32_t nMeshes, uint32_t n, int bits)
     o = align256(o + sizeof(uint32_t) * (size_t)nMeshes * passes * bins);
     L.lookback = o;
     o = align256(o + sizeof(uint32_t) * (size_t)passes * L.maxTiles * bins);
+    L.treeCounts = o;
+    o = align256(o + tree::count_bytes(n));
     L.zeroEnd = o;
     L.keysA = o;
     o = align256(o + sizeof(uint32_t) * (size_t)n);
@@ -97,6 +102,8 @@ BatchLayout batch_layout(uint32_t nMeshes, uint32_t n, int bits)
     o = align256(o + sizeof(uint32_t) * (size_t)n);
     L.handoff = o;
     o = align256(o + sizeof(uint32_t) * (size_t)n);
+    L.summary = o;
+    o = align256(o + tree::summary_bytes(n));
     L.total = o;
     return L;
 }
@@ -191,7 +198,10 @@ __global__ void __launch_bounds__(kPlanThreads)
     }
     if (threadIdx.x == 0) {
         tileStart[nMeshes] = running;
-        if (bad) header[kHdrError] = kErrOffsets;
+        if (bad) {
+            header[kHdrError] = kErrOffsets;
+            header[kHdrTreeFlags] = tree::kSkip;
+        }
     }
     for (uint32_t i = threadIdx.x; i < 6 * nMeshes; i += kPlanThreads) bounds[i] = (i % 6) < 3 ? 0xFFFFFFFFu : 0u;
 }
@@ -307,7 +317,7 @@ __global__ void __launch_bounds__(kTileThreads)
     k_batch_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const uint32_t* __restrict__ off,
                  uint32_t nMeshes, const uint32_t* __restrict__ tileStart, const uint32_t* __restrict__ bounds,
                  uint32_t* __restrict__ keys, uint32_t* __restrict__ histogram, uint32_t* __restrict__ handoff,
-                 mlbvh_aabb* __restrict__ meshAABBs)
+                 mlbvh_aabb* __restrict__ meshAABBs, uint32_t* __restrict__ treeFlags)
 {
     using S = sort::Shape<kBits>;
     constexpr int kBins = S::kBins, kPasses = S::kPasses;
@@ -336,6 +346,7 @@ __global__ void __launch_bounds__(kTileThreads)
             const float* t = s_tri + 9 * threadIdx.x;
             f3 v0 = mk(t[0], t[1], t[2]), v1 = mk(t[3], t[4], t[5]), v2 = mk(t[6], t[7], t[8]);
             f3 center = (v0 + v1 + v2) / 3.0f;
+            if (isnan(center.x) || isnan(center.y) || isnan(center.z)) atomicOr(treeFlags, tree::kNaN);
             uint32_t key;
             if (option & MLBVH_BUILD_OPTION_USE_NORMAL) {
                 f3 ng = normalize(cross(v1 - v0, v2 - v0));
@@ -359,38 +370,19 @@ __global__ void __launch_bounds__(kTileThreads)
 }
 
 
-// build_lbvh (minimum_lbvh.h:284-361), one thread per sorted leaf: the tile
-// climb of the single-mesh build, over tiles of kTileLeaves consecutive leaves
-// of the whole batch. A tile may hold the end of one mesh and the start of the
-// next: the delta across a mesh boundary is staged as infinite (the value each
-// mesh's climb gives the deltas outside its range), so each node's range, and
-// with it its interior test, stays inside its mesh.
-static_assert(kBuildThreads == (int)kTileLeaves, "one thread per leaf of a tile");
-__global__ void __launch_bounds__(kBuildThreads)
-    k_batch_build(const float* __restrict__ tris, uint32_t n, const uint32_t* __restrict__ off, uint32_t nMeshes,
-                  const uint32_t* __restrict__ sortedKeys, const uint32_t* __restrict__ sortedIdx,
-                  mlbvh_internal_node* __restrict__ allNodes, uint32_t* __restrict__ allHandoff,
-                  mlbvh_node_index* __restrict__ roots, const uint32_t* __restrict__ header)
-{
-    __shared__ TileClimbShared sh;
-    if (__ldcg(header + kHdrError) & kErrOffsets) return;  // the whole CTA: the plan's word is set before
-    const uint32_t t0 = blockIdx.x * kTileLeaves;
-    const uint32_t g = t0 + threadIdx.x;
-    uint32_t m = 0, start = n, end = n, tri = 0xFFFFFFFFu;
-    f3 lo = mk(0.0f, 0.0f, 0.0f), hi = lo;
-    if (g < n) {
-        m = find_segment(off, nMeshes, g);
-        start = __ldg(off + m);
-        end = __ldg(off + m + 1);
-        tri = sortedIdx[g];
-        // tri >= the mesh's size only after a sort whose bounded wait gave up (error word set)
-        if (tri < end - start) leaf_box(tris + 9 * (size_t)start, end - start, tri, lo, hi);
+// The batch's trees for tree.cuh: mesh m's leaves are [off[m], off[m + 1]).
+struct MeshTrees {
+    static constexpr bool kMany = true;
+    const uint32_t* off;
+    uint32_t nMeshes;
+    __device__ __forceinline__ tree::Segment of(uint32_t g) const
+    {
+        const uint32_t m = find_segment(off, nMeshes, g);
+        return tree::Segment{__ldg(off + m), __ldg(off + m + 1), m};
     }
-    tile_climb_prepare(sh, sortedKeys, n, t0, start, end);
-    if (g >= n || tri >= end - start) return;
-    climb_tile(sh, t0 - start, end - start, g - start, tri, lo, hi, sortedKeys + start, allNodes + (start - m),
-               allHandoff + (start - m), roots + m, nullptr);
-}
+    __device__ __forceinline__ uint32_t start_of(uint32_t m) const { return __ldg(off + m); }
+    __device__ __forceinline__ uint32_t end_of(uint32_t m) const { return __ldg(off + m + 1); }
+};
 
 // The persistent traversal (see the file comment). Hits are written as
 // mlbvh_trace writes them; ray i of the batch belongs to the mesh m with
@@ -553,7 +545,8 @@ mlbvh_status launch_build(const mlbvh_batch& B, const BatchLayout& L, cudaStream
     k_batch_bounds<<<L.maxTiles, kTileThreads, 0, stream>>>(tris, n, off, nm, tileStart, bounds, hist, zeroWords);
     MLBVH_CHECK_LAUNCH("k_batch_bounds");
     k_batch_keys<kBits><<<L.maxTiles, kTileThreads, 0, stream>>>(tris, n, B.buildOption, off, nm, tileStart, bounds,
-                                                                 keysA, hist, handoff, B.dMeshAABBs);
+                                                                 keysA, hist, handoff, B.dMeshAABBs,
+                                                                 header + kHdrTreeFlags);
     MLBVH_CHECK_LAUNCH("k_batch_keys");
     uint32_t* kin = keysA;
     uint32_t* vin = valsA;
@@ -574,9 +567,12 @@ mlbvh_status launch_build(const mlbvh_batch& B, const BatchLayout& L, cudaStream
     }
     const ProfileEvents ev = take_profile_events();
     if (ev.start) cudaEventRecord(ev.start, stream);
-    k_batch_build<<<(n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, stream>>>(
-        tris, n, off, nm, kin, vin, B.dInternals, handoff, B.dRootNodes, header);
-    MLBVH_CHECK_LAUNCH("k_batch_build");
+    // the buffers the last pass read are free
+    const tree::Scratch sc = tree::place(n, s + L.summary, reinterpret_cast<uint32_t*>(s + L.treeCounts),
+                                         header + kHdrTreeFlags, kin == keysA ? keysB : keysA);
+    if (mlbvh_status st = tree::launch(tris, MeshTrees{off, nm}, kin, vin, B.dInternals, B.dRootNodes, nullptr,
+                                       handoff, sc, device_sm_count(), stream))
+        return st;
     if (ev.stop) cudaEventRecord(ev.stop, stream);
     return MLBVH_OK;
 }

@@ -13,8 +13,8 @@
 //   k_onesweep x4    one stable pass per digit: warp multisplit, decoupled
 //                    look-back over per-tile digit counts, scatter through
 //                    shared memory so that runs of one digit store coalesced
-//   k_build          one thread per sorted leaf climbs to the root
-//                    (build_lbvh, minimum_lbvh.h:284-361)
+//   k_tree_tiles, k_tree_cross   the tree (build_lbvh, minimum_lbvh.h:284-361;
+//                    tree.cuh)
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -23,6 +23,8 @@
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
+#include "sort_leaves.cuh"
+#include "tree.cuh"
 
 namespace mlbvh {
 
@@ -32,19 +34,20 @@ constexpr int kBoundsThreads = 256;
 constexpr int kBoundsMaxBlocks = 1024;
 constexpr int kKeysThreads = 256;
 constexpr int kSortTile = sort::kTile;  // 4096 keys per tile
-constexpr int kBuildThreads = (int)kTileLeaves;
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
+constexpr int kHdrTreeFlags = 5;  // header word of tree::Scratch::flags; the record count follows
 
 // Scratch layout of one build (offsets from the caller's dScratch). The
 // leading region [header, partials) is zeroed by k_scene_bounds on every build.
 struct BuildLayout {
-    size_t header;     // u32 error word, u32 tile counters[4]
+    size_t header;     // u32 error word, u32 tile counters[4], u32 tree flags, u32 tree records
     size_t histogram;  // 4 x 256 u32
     size_t lookback;   // 4 x tiles x 256 u32
+    size_t treeCounts; // tree::count_bytes(n)
     size_t partials;   // kBoundsMaxBlocks x 8 floats
     size_t keysA, keysB, valsA, valsB;
     size_t handoff;  // n u32
-    size_t deltas;   // n u8
+    size_t summary;  // tree::summary_bytes(n)
     size_t total;
     uint32_t tiles;
 };
@@ -62,6 +65,8 @@ BuildLayout build_layout(uint32_t n)
     o = align256(o + sizeof(uint32_t) * 4 * 256);
     L.lookback = o;
     o = align256(o + sizeof(uint32_t) * 4 * 256 * (size_t)L.tiles);
+    L.treeCounts = o;
+    o = align256(o + tree::count_bytes(n));
     L.partials = o;
     o = align256(o + sizeof(float) * 8 * kBoundsMaxBlocks);
     L.keysA = o;
@@ -74,8 +79,8 @@ BuildLayout build_layout(uint32_t n)
     o = align256(o + sizeof(uint32_t) * (size_t)n);
     L.handoff = o;
     o = align256(o + sizeof(uint32_t) * (size_t)n);
-    L.deltas = o;
-    o = align256(o + (size_t)n);
+    L.summary = o;
+    o = align256(o + tree::summary_bytes(n));
     L.total = o;
     return L;
 }
@@ -144,7 +149,7 @@ __global__ void __launch_bounds__(kBoundsThreads)
 __global__ void __launch_bounds__(kKeysThreads)
     k_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const float* __restrict__ partials,
            int nPartials, uint32_t* __restrict__ keys, uint32_t* __restrict__ histogram,
-           uint32_t* __restrict__ handoff, mlbvh_aabb* __restrict__ sceneOut)
+           uint32_t* __restrict__ handoff, mlbvh_aabb* __restrict__ sceneOut, uint32_t* __restrict__ treeFlags)
 {
     __shared__ float s_scene[6];
     __shared__ uint32_t s_hist[4][256];
@@ -196,6 +201,7 @@ __global__ void __launch_bounds__(kKeysThreads)
             const float* t = s_tri + threadIdx.x * 9;
             f3 v0 = mk(t[0], t[1], t[2]), v1 = mk(t[3], t[4], t[5]), v2 = mk(t[6], t[7], t[8]);
             f3 center = (v0 + v1 + v2) / 3.0f;
+            if (isnan(center.x) || isnan(center.y) || isnan(center.z)) atomicOr(treeFlags, tree::kNaN);
             uint32_t key;
             if (option & MLBVH_BUILD_OPTION_USE_NORMAL) {
                 f3 ng = normalize(cross(v1 - v0, v2 - v0));
@@ -217,34 +223,13 @@ __global__ void __launch_bounds__(kKeysThreads)
     }
 }
 
-
-// One thread per sorted leaf of the single-mesh build, one CTA per tile of
-// kTileLeaves leaves (climb_tile: the tile's own nodes meet in shared memory).
-static_assert(kBuildThreads == (int)kTileLeaves, "one thread per leaf of a tile");
-__global__ void __launch_bounds__(kBuildThreads)
-    k_build(const float* __restrict__ tris, uint32_t n, const uint32_t* __restrict__ sortedKeys,
-            const uint32_t* __restrict__ sortedIdx, mlbvh_internal_node* __restrict__ nodes,
-            uint32_t* __restrict__ handoff, mlbvh_node_index* __restrict__ root, uint8_t* __restrict__ deltas)
-{
-    __shared__ TileClimbShared sh;
-    const uint32_t t0 = blockIdx.x * kTileLeaves;
-    const uint32_t i = t0 + threadIdx.x;
-    // tri >= n only after a sort whose bounded wait gave up (error word set)
-    const uint32_t tri = i < n ? sortedIdx[i] : 0xFFFFFFFFu;
-    f3 lo = mk(0.0f, 0.0f, 0.0f), hi = lo;
-    if (tri < n) leaf_box(tris, n, tri, lo, hi);
-    tile_climb_prepare(sh, sortedKeys, n, t0, 0u, n);
-    if (tri >= n) return;
-    climb_tile(sh, t0, n, i, tri, lo, hi, sortedKeys, nodes, handoff, root, deltas);
-}
-
 }  // namespace
 
 size_t build_scratch_bytes(uint32_t n) { return build_layout(n).total; }
 
 mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t option, mlbvh_aabb* dScene,
-                         uint32_t* dKeysOut, uint32_t* dIdxOut, uint8_t* dDeltasOut, void* dScratch,
-                         cudaStream_t stream, uint32_t spinLimit, SortedLeaves* out)
+                         uint32_t* dKeysOut, uint32_t* dIdxOut, void* dScratch, cudaStream_t stream,
+                         uint32_t spinLimit, SortedLeaves* out)
 {
     const BuildLayout L = build_layout(n);
     if (spinLimit == 0) spinLimit = kDefaultSpinLimit;
@@ -271,7 +256,7 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
     MLBVH_CHECK_LAUNCH("k_scene_bounds");
     const int keysBlocks = std::max(1, std::min<int>((n + kKeysThreads - 1) / kKeysThreads, 8 * sms));
     k_keys<<<keysBlocks, kKeysThreads, 0, stream>>>(tris, n, option, partials, boundsBlocks, keysA, hist, handoff,
-                                                    dScene);
+                                                    dScene, header + kHdrTreeFlags);
     MLBVH_CHECK_LAUNCH("k_keys");
 
     uint32_t* kin = keysA;
@@ -298,7 +283,9 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
     out->indices = valsFinal;
     out->error = header;
     out->handoff = handoff;
-    out->deltas = dDeltasOut ? dDeltasOut : reinterpret_cast<uint8_t*>(s + L.deltas);
+    // after four passes the last pass's inputs are free
+    out->tree = tree::place(n, s + L.summary, reinterpret_cast<uint32_t*>(s + L.treeCounts), header + kHdrTreeFlags,
+                               keysB);
     out->spinLimit = spinLimit;
     return MLBVH_OK;
 }
@@ -316,14 +303,13 @@ mlbvh_status build(const mlbvh_triangle* dTris, uint32_t n, uint32_t option, mlb
     if (scratchBytes < build_layout(n).total)
         return fail(MLBVH_ERR_INVALID_ARG, "scratch smaller than mlbvh_build_scratch_bytes(n)");
     SortedLeaves sl;
-    mlbvh_status st = sort_leaves(dTris, n, option, dScene, dKeysOut, dIdxOut, dDeltasOut, dScratch, stream,
-                                  spinLimit, &sl);
+    mlbvh_status st = sort_leaves(dTris, n, option, dScene, dKeysOut, dIdxOut, dScratch, stream, spinLimit, &sl);
     if (st != MLBVH_OK) return st;
     ProfileEvents ev = take_profile_events();
     if (ev.start) cudaEventRecord(ev.start, stream);
-    k_build<<<(n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, stream>>>(
-        reinterpret_cast<const float*>(dTris), n, sl.keys, sl.indices, dNodes, sl.handoff, dRoot, sl.deltas);
-    MLBVH_CHECK_LAUNCH("k_build");
+    st = tree::launch(reinterpret_cast<const float*>(dTris), tree::OneTree{n}, sl.keys, sl.indices, dNodes, dRoot,
+                      dDeltasOut, sl.handoff, sl.tree, device_sm_count(), stream);
+    if (st != MLBVH_OK) return st;
     if (ev.stop) cudaEventRecord(ev.stop, stream);
     return MLBVH_OK;
 }

@@ -59,6 +59,7 @@
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
+#include "sort_leaves.cuh"
 
 namespace mlbvh {
 
@@ -800,7 +801,7 @@ mlbvh_status build_ploc(const mlbvh_triangle* dTris, uint32_t n, uint32_t option
                      stream, spinLimit);
 
     SortedLeaves sl;
-    mlbvh_status st = sort_leaves(dTris, n, option, dScene, nullptr, nullptr, nullptr, dScratch, stream, spinLimit, &sl);
+    mlbvh_status st = sort_leaves(dTris, n, option, dScene, nullptr, nullptr, dScratch, stream, spinLimit, &sl);
     if (st != MLBVH_OK) return st;
 
     char* s = static_cast<char*>(dScratch);
