@@ -33,7 +33,14 @@ namespace {
 constexpr int kBoundsThreads = 256;
 constexpr int kBoundsMaxBlocks = 1024;
 constexpr int kKeysThreads = 256;
-constexpr int kSortTile = sort::kTile;  // 4096 keys per tile
+// Arrays whose tiles of 1024 keys are all resident at once (3 CTAs on each of
+// 148 multiprocessors) sort in those instead of tiles of 4096: a tile's time
+// is the chain of its rank steps, and more tiles share the work. Whole builds
+// with 1024 / 4096 keys a tile: 16,000 triangles 59 / 73 us, 65,000 72 / 85,
+// 213,000 93 / 100, 450,000 124 / 127; beyond, the second wave costs more. The
+// small tiles look back 4 at a time (213,000: 1 at a time 100 us, 8 93, 16 93;
+// 450,000: 136, 126, 129).
+constexpr uint32_t kFewMax = 3 * 148 * sort::kThreads * sort::kFewItems;
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
 constexpr int kHdrTreeFlags = 5;  // header word of tree::Scratch::flags; the record count follows
 
@@ -57,7 +64,8 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 BuildLayout build_layout(uint32_t n)
 {
     BuildLayout L;
-    L.tiles = (n + kSortTile - 1) / kSortTile;
+    const uint32_t sortTile = sort::kThreads * (n <= kFewMax ? sort::kFewItems : sort::kItems);
+    L.tiles = (n + sortTile - 1) / sortTile;
     size_t o = 0;
     L.header = o;
     o += 256;
@@ -143,9 +151,24 @@ __global__ void __launch_bounds__(kBoundsThreads)
     }
 }
 
-// Morton key per triangle (buildMortons, minimum_lbvh.cu:68-92) plus the four
-// digit histograms of the sort. Triangles are staged through shared memory
-// with 16-byte loads, 256 triangles (2304 floats) per step.
+// The Morton key of a triangle (buildMortons, minimum_lbvh.cu:68-92).
+__device__ __forceinline__ uint32_t triangle_key(const float* t, uint32_t option, f3 lower, f3 upper,
+                                                 uint32_t* __restrict__ treeFlags)
+{
+    const f3 v0 = mk(t[0], t[1], t[2]), v1 = mk(t[3], t[4], t[5]), v2 = mk(t[6], t[7], t[8]);
+    const f3 center = (v0 + v1 + v2) / 3.0f;
+    if (isnan(center.x) || isnan(center.y) || isnan(center.z)) atomicOr(treeFlags, tree::kNaN);
+    const uint32_t key = morton32(lower, upper, center);
+    if (!(option & MLBVH_BUILD_OPTION_USE_NORMAL)) return key;
+    const f3 ng = normalize(cross(v1 - v0, v2 - v0));
+    return (key & 0xFFFFFFC0u) | (morton32(mk(-1, -1, -1), mk(1, 1, 1), ng) >> 26);
+}
+
+// The keys of all triangles plus the four digit histograms of the sort. A
+// warp takes 32 triangles at a time through its own shared memory with
+// coalesced 16-byte loads, the next 32 already on their way, last triangles
+// first: the bounds pass has just read the array forwards, so its end is what
+// the L2 still holds.
 __global__ void __launch_bounds__(kKeysThreads)
     k_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const float* __restrict__ partials,
            int nPartials, uint32_t* __restrict__ keys, uint32_t* __restrict__ histogram,
@@ -153,17 +176,42 @@ __global__ void __launch_bounds__(kKeysThreads)
 {
     __shared__ float s_scene[6];
     __shared__ uint32_t s_hist[4][256];
-    __shared__ __align__(16) float s_tri[kKeysThreads * 9];  // written with 16-byte stores
+    __shared__ float4 s_tri[kKeysThreads / 32][72];  // 32 triangles of 9 floats per warp
+
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t chunks = (n + 31) / 32, warps = gridDim.x * (kKeysThreads / 32);
+    float4 ahead[3];
+    auto load = [&](uint32_t c) {  // words 4 lane, 4 lane + 128 and (lanes 0..7) 4 lane + 256 of chunk c
+        const size_t base = (size_t)c * 288, words = (size_t)n * 9;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const size_t w = base + 4 * lane + 128 * k;
+            if (k == 2 && lane >= 8) break;
+            if (w + 4 <= words) {
+                ahead[k] = __ldg(reinterpret_cast<const float4*>(tris + w));
+            } else {
+                float* x = reinterpret_cast<float*>(&ahead[k]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = w + j < words ? __ldg(tris + w + j) : 0.0f;
+            }
+        }
+    };
+    uint32_t c = blockIdx.x * (kKeysThreads / 32) + warp;  // counted from the last chunk
+    if (c < chunks) load(chunks - 1 - c);
 
     for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
+    if (warp == 0) {
         float lo[3] = {kFltMax, kFltMax, kFltMax}, hi[3] = {-kFltMax, -kFltMax, -kFltMax};
-        for (int p = lane; p < nPartials; p += 32)
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fminf(lo[a], partials[p * 8 + a]);
-                hi[a] = fmaxf(hi[a], partials[p * 8 + 3 + a]);
+        for (int p = lane; p < nPartials; p += 32) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(partials + p * 8));
+            const float4 b = __ldg(reinterpret_cast<const float4*>(partials + p * 8) + 1);
+            const float l[3] = {a.x, a.y, a.z}, h[3] = {a.w, b.x, b.y};
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                lo[x] = fminf(lo[x], l[x]);
+                hi[x] = fmaxf(hi[x], h[x]);
             }
+        }
         for (int o = 16; o > 0; o >>= 1)
             for (int a = 0; a < 3; ++a) {
                 lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
@@ -183,35 +231,19 @@ __global__ void __launch_bounds__(kKeysThreads)
     const f3 lower = mk(s_scene[0], s_scene[1], s_scene[2]);
     const f3 upper = mk(s_scene[3], s_scene[4], s_scene[5]);
 
-    const size_t gthreads = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i + 1 < n; i += gthreads) handoff[i] = 0xFFFFFFFFu;
-
-    const uint32_t nTiles = (n + kKeysThreads - 1) / kKeysThreads;
-    for (uint32_t tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
-        const size_t fbase = (size_t)tile * kKeysThreads * 9;
-        const size_t fcount = min((size_t)kKeysThreads * 9, (size_t)n * 9 - fbase);
-        const float4* src4 = reinterpret_cast<const float4*>(tris + fbase);
-        const int n4 = (int)(fcount / 4);
-        __syncthreads();
-        for (int j = threadIdx.x; j < n4; j += kKeysThreads) reinterpret_cast<float4*>(s_tri)[j] = __ldg(src4 + j);
-        for (int j = n4 * 4 + threadIdx.x; j < (int)fcount; j += kKeysThreads) s_tri[j] = __ldg(tris + fbase + j);
-        __syncthreads();
-        const uint32_t i = tile * kKeysThreads + threadIdx.x;
+    for (; c < chunks; c += warps) {
+        const uint32_t chunk = chunks - 1 - c, i = chunk * 32 + lane;
+        __syncwarp();
+        s_tri[warp][lane] = ahead[0];
+        s_tri[warp][lane + 32] = ahead[1];
+        if (lane < 8) s_tri[warp][lane + 64] = ahead[2];
+        __syncwarp();
+        if (c + warps < chunks) load(chunks - 1 - c - warps);
         if (i < n) {
-            const float* t = s_tri + threadIdx.x * 9;
-            f3 v0 = mk(t[0], t[1], t[2]), v1 = mk(t[3], t[4], t[5]), v2 = mk(t[6], t[7], t[8]);
-            f3 center = (v0 + v1 + v2) / 3.0f;
-            if (isnan(center.x) || isnan(center.y) || isnan(center.z)) atomicOr(treeFlags, tree::kNaN);
-            uint32_t key;
-            if (option & MLBVH_BUILD_OPTION_USE_NORMAL) {
-                f3 ng = normalize(cross(v1 - v0, v2 - v0));
-                uint32_t nMorton = morton32(mk(-1, -1, -1), mk(1, 1, 1), ng);
-                uint32_t pMorton = morton32(lower, upper, center);
-                key = (pMorton & 0xFFFFFFC0u) | (nMorton >> 26);
-            } else {
-                key = morton32(lower, upper, center);
-            }
+            const uint32_t key = triangle_key(reinterpret_cast<const float*>(s_tri[warp]) + 9 * lane, option, lower,
+                                              upper, treeFlags);
             keys[i] = key;
+            handoff[i] = 0xFFFFFFFFu;
 #pragma unroll
             for (int d = 0; d < 4; ++d) atomicAdd(&s_hist[d][(key >> (8 * d)) & 255u], 1u);
         }
@@ -249,32 +281,33 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
 
     const int sms = device_sm_count();
     const size_t zeroWords = (L.partials - L.header) / 4;
-    int boundsBlocks = (int)std::min<size_t>((size_t)kBoundsMaxBlocks,
-                                             std::max<size_t>(1, ((size_t)n * 9 / 12 + kBoundsThreads - 1) / kBoundsThreads));
+    // at least four vertex groups per thread, and four warp chunks per warp of k_keys: both kernels end in a
+    // reduction over their CTAs
+    int boundsBlocks = (int)std::min<size_t>(
+        (size_t)kBoundsMaxBlocks, std::max<size_t>(1, ((size_t)n * 9 / 48 + kBoundsThreads - 1) / kBoundsThreads));
     boundsBlocks = std::min(boundsBlocks, 4 * sms);
     k_scene_bounds<<<boundsBlocks, kBoundsThreads, 0, stream>>>(tris, n, partials, header, zeroWords);
     MLBVH_CHECK_LAUNCH("k_scene_bounds");
-    const int keysBlocks = std::max(1, std::min<int>((n + kKeysThreads - 1) / kKeysThreads, 8 * sms));
+    const int keysBlocks = (int)std::max<uint32_t>(1, std::min<uint32_t>((n + 4 * kKeysThreads - 1) / (4 * kKeysThreads), 4u * sms));
     k_keys<<<keysBlocks, kKeysThreads, 0, stream>>>(tris, n, option, partials, boundsBlocks, keysA, hist, handoff,
                                                     dScene, header + kHdrTreeFlags);
     MLBVH_CHECK_LAUNCH("k_keys");
 
     uint32_t* kin = keysA;
     uint32_t* vin = valsA;
-    constexpr size_t kSmem = sort::Shape<8>::kSmemBytes;
+    const bool few = n <= kFewMax;
+    const size_t smem = few ? sort::Shape<8, sort::kFewItems>::kSmemBytes : sort::Shape<8>::kSmemBytes;
     for (int pass = 0; pass < 4; ++pass) {
         uint32_t* kout = (pass == 3) ? keysFinal : (pass % 2 == 0 ? keysB : keysA);
         uint32_t* vout = (pass == 3) ? valsFinal : (pass % 2 == 0 ? valsB : valsA);
         const sort::SingleSegment seg{n, L.tiles, hist + 256 * pass};
-        uint32_t* lb = lookback + (size_t)pass * L.tiles * 256;
-        if (pass == 0)
-            sort::k_onesweep<8, true><<<L.tiles, sort::kThreads, kSmem, stream>>>(kin, kout, nullptr, vout, 8 * pass,
-                                                                                seg, lb, header + 1 + pass, header,
-                                                                                spinLimit);
-        else
-            sort::k_onesweep<8, false><<<L.tiles, sort::kThreads, kSmem, stream>>>(kin, kout, vin, vout, 8 * pass,
-                                                                                 seg, lb, header + 1 + pass, header,
-                                                                                 spinLimit);
+        using Seg = sort::SingleSegment;
+        auto kernel = few ? (pass == 0 ? sort::k_onesweep<8, true, Seg, sort::kFewItems>
+                                       : sort::k_onesweep<8, false, Seg, sort::kFewItems>)
+                          : (pass == 0 ? sort::k_onesweep<8, true, Seg> : sort::k_onesweep<8, false, Seg>);
+        kernel<<<L.tiles, sort::kThreads, smem, stream>>>(kin, kout, pass == 0 ? nullptr : vin, vout, 8 * pass, seg,
+                                                          lookback + (size_t)pass * L.tiles * 256, header + 1 + pass,
+                                                          header, spinLimit);
         MLBVH_CHECK_LAUNCH("k_onesweep");
         kin = kout;
         vin = vout;

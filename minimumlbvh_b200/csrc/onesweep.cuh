@@ -29,11 +29,13 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096 keys per tile
+constexpr int kFewItems = 4;              // small arrays: 1024 keys per tile
+constexpr uint32_t kWindow = 4;  // earlier tiles per look-back step of the small tiles (1, 8, 16: see build.cu)
 constexpr uint32_t kFlagAggregate = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1;
 
-template <int kBits>
+template <int kBits, int kPer = kItems>
 struct Shape {
     static_assert(kBits == 8 || kBits == 11, "digit width must be 8 or 11 bits");
     static constexpr int kBins = 1 << kBits;
@@ -41,7 +43,7 @@ struct Shape {
     static constexpr int kPasses = (32 + kBits - 1) / kBits;
     // dynamic shared memory: per-warp digit counts (reused for the scatter
     // destinations), tile-exclusive digit offsets, staged keys and values
-    static constexpr size_t kSmemBytes = sizeof(uint32_t) * ((size_t)kWarps * kBins + kBins + 2 * (size_t)kTile);
+    static constexpr size_t kSmemBytes = sizeof(uint32_t) * ((size_t)kWarps * kBins + kBins + 2 * (size_t)kThreads * kPer);
 };
 
 // One segment as a tile sees it.
@@ -52,7 +54,7 @@ struct Segment {
     const uint32_t* counts;    // the segment's digit counts for this pass (kBins)
 };
 
-// The whole array is one segment of n keys; tile ids 0 .. ceil(n / kTile) - 1.
+// The whole array is one segment of n keys; tile ids 0 .. tiles - 1.
 struct SingleSegment {
     uint32_t n;
     uint32_t tiles;
@@ -140,15 +142,17 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp /*kW
 // are held to three resident CTAs per SM (at most 85 registers): the pass is
 // latency-bound and more tiles in flight shorten it (measured 3 % on a 4M
 // build); the 11-bit passes are limited by shared memory to two anyway.
-template <int kBits, bool kFirst, class Segments>
+// kPer keys per thread: the rank chain of a tile is kPer steps long, so an
+// array that leaves multiprocessors idle is cut into smaller tiles.
+template <int kBits, bool kFirst, class Segments, int kPer = kItems>
 __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
     k_onesweep(const uint32_t* __restrict__ keysIn, uint32_t* __restrict__ keysOut,
                const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ valsOut, int shift, Segments segs,
                uint32_t* __restrict__ lookback, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ errorWord,
                uint32_t spinLimit)
 {
-    using S = Shape<kBits>;
-    constexpr int kBins = S::kBins, kDPT = S::kDigitsPerThread;
+    using S = Shape<kBits, kPer>;
+    constexpr int kBins = S::kBins, kDPT = S::kDigitsPerThread, kTile = kThreads * kPer;
     constexpr uint32_t kMask = (uint32_t)kBins - 1u;
     extern __shared__ __align__(16) uint32_t smem[];
     uint32_t* s_warpHist = smem;                  // [kWarps][kBins]
@@ -187,10 +191,10 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
         }
     }
 
-    const uint32_t localBase = chunk * (uint32_t)kTile + (uint32_t)warp * (kItems * 32);
-    uint32_t key[kItems], val[kItems], rank[kItems];
+    const uint32_t localBase = chunk * (uint32_t)kTile + (uint32_t)warp * (kPer * 32);
+    uint32_t key[kPer], val[kPer], rank[kPer];
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
+    for (int k = 0; k < kPer; ++k) {
         const uint32_t li = localBase + k * 32 + lane;
         const bool valid = li < seg.len;
         key[k] = valid ? __ldg(keysIn + seg.start + li) : 0xFFFFFFFFu;
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
     const uint32_t lanesBelow = (1u << lane) - 1u;
     uint32_t* myHist = s_warpHist + warp * kBins;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
+    for (int k = 0; k < kPer; ++k) {
         const uint32_t li = localBase + k * 32 + lane;
         const uint32_t d = (key[k] >> shift) & kMask;
         uint32_t peers = __ballot_sync(0xffffffffu, li < seg.len);
@@ -239,7 +243,37 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
         st_relaxed(lookback + (size_t)tile * kBins + j * kThreads + tid,
                    (chunk == 0 ? kFlagPrefix : kFlagAggregate) | count[j]);
     }
-    if (chunk != 0) {
+    if constexpr (kPer == kFewItems) {
+        // Many small tiles: a thread reads the words of kWindow earlier tiles
+        // at once and takes those that are ready from the nearest on, one L2
+        // round trip per kWindow tiles instead of one per tile.
+        bool done = chunk == 0;
+        uint32_t left = chunk, spins = 0;  // earlier tiles not yet counted
+        while (!done) {
+            const uint32_t* row = lookback + ((size_t)tile - chunk + left) * kBins + tid;
+            uint32_t w[kWindow];
+#pragma unroll
+            for (uint32_t i = 0; i < kWindow; ++i)
+                w[i] = i < left ? ld_relaxed(row - (size_t)(i + 1) * kBins) : kFlagPrefix;
+            uint32_t taken = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < kWindow; ++i)
+                if (!done && taken == i && (w[i] >> 30) != 0u) {
+                    prefix[0] += w[i] & kValueMask;
+                    done = (w[i] >> 30) == 2u;
+                    ++taken;
+                }
+            left -= min(taken, left);
+            if (taken) {
+                spins = 0;
+            } else if (++spins > spinLimit) {
+                atomicOr(errorWord, 1u);
+                done = true;
+            } else {
+                __nanosleep(20);
+            }
+        }
+    } else if (chunk != 0) {
         uint32_t done = 0;
         constexpr uint32_t kAll = (1u << kDPT) - 1u;
         for (uint32_t t = tile - 1;; --t) {
@@ -273,6 +307,8 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
                 }
             if (done == kAll || t == seg.firstTile) break;
         }
+    }
+    if (chunk != 0) {
 #pragma unroll
         for (int j = 0; j < kDPT; ++j)
             st_relaxed(lookback + (size_t)tile * kBins + j * kThreads + tid,
@@ -297,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
 
     // place every key at its tile-sorted position in shared memory
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
+    for (int k = 0; k < kPer; ++k) {
         const uint32_t li = localBase + k * 32 + lane;
         if (li < seg.len) {
             const uint32_t dk = (key[k] >> shift) & kMask;
