@@ -316,6 +316,81 @@ struct ReplayStack<true> {
 // walk to stackfree_step at (near child, this node), marked by depth = -1;
 // climbing through the parent links, it re-derives every entry still on the
 // stack. Start a walk with curr = root, depth = 0.
+//
+// replay_leaf tests the leaf curr (true: an any-hit walk is over), replay_node
+// visits the node curr (true: curr is the next node or leaf), replay_pop takes
+// the next pending entry (true: none is left); stackfree_replay_step makes one
+// step of them, and a kernel that schedules leaf tests itself calls them.
+template <bool kAny>
+__device__ __forceinline__ bool replay_leaf(uint32_t curr, HitRecord& hit, const float* __restrict__ tris, f3 ro, f3 rd,
+                                            float tmin)
+{
+    const uint32_t ti = curr & ~kLeafBit;
+    f3 v0, v1, v2;
+    load_triangle(tris, ti, v0, v1, v2);
+    float t, u, v;
+    f3 ng;
+    if (intersect_triangle(t, u, v, ng, tmin, hit.t, ro, rd, v0, v1, v2)) {
+        hit.t = t;
+        hit.u = u;
+        hit.v = v;
+        hit.ng = ng;
+        hit.tri = ti;
+        return kAny;
+    }
+    return false;
+}
+template <bool kAny, int kDepth>
+__device__ __forceinline__ bool replay_node(uint32_t& curr, uint32_t& prev, int& depth,
+                                            typename ReplayStack<kAny>::Entry* stack, int stride, float hitT,
+                                            const mlbvh_internal_node* __restrict__ nodes, f3 ro, f3 inv, float tmin)
+{
+    const NodeView nd = load_node<true>(nodes, curr);
+    const float2 rl = slab(ro, inv, nd.lo0, nd.hi0, tmin, hitT);
+    const float2 rr = slab(ro, inv, nd.lo1, nd.hi1, tmin, hitT);
+    const bool hitL = rl.x <= rl.y, hitR = rr.x <= rr.y;
+    if (hitL && hitR) {
+        const bool swap = rr.x < rl.x;
+        const uint32_t nearN = swap ? nd.c1 : nd.c0, farN = swap ? nd.c0 : nd.c1;
+        if (depth == kDepth) {  // full: continue as the stack-free walk
+            depth = -1;
+            prev = curr;
+            curr = nearN;
+            return true;
+        }
+        if constexpr (kAny)
+            stack[depth * stride] = farN;
+        else
+            stack[depth * stride] = make_uint2(farN, __float_as_uint(swap ? rl.x : rr.x));
+        ++depth;
+        curr = nearN;
+        return true;
+    }
+    if (hitL || hitR) {
+        curr = hitL ? nd.c0 : nd.c1;
+        return true;
+    }
+    return false;
+}
+template <bool kAny>
+__device__ __forceinline__ bool replay_pop(uint32_t& curr, int& depth, typename ReplayStack<kAny>::Entry* stack,
+                                           int stride, float hitT)
+{
+    if constexpr (kAny) {
+        if (depth == 0) return true;
+        curr = stack[--depth * stride];
+        return false;
+    } else {
+        while (depth > 0) {
+            const uint2 e = stack[--depth * stride];
+            if (__uint_as_float(e.y) <= hitT) {
+                curr = e.x;
+                return false;
+            }
+        }
+        return true;
+    }
+}
 template <bool kAny, bool kCount, int kDepth>
 __device__ __forceinline__ bool stackfree_replay_step(uint32_t& curr, uint32_t& prev, int& depth,
                                                       typename ReplayStack<kAny>::Entry* stack,
@@ -327,61 +402,12 @@ __device__ __forceinline__ bool stackfree_replay_step(uint32_t& curr, uint32_t& 
     if (depth < 0) return stackfree_step<kAny, kCount, true>(curr, prev, hit, nodes, tris, ro, rd, inv, tmin, nv, nt);
     if (curr & kLeafBit) {
         if (kCount) ++nt;
-        const uint32_t ti = curr & ~kLeafBit;
-        f3 v0, v1, v2;
-        load_triangle(tris, ti, v0, v1, v2);
-        float t, u, v;
-        f3 ng;
-        if (intersect_triangle(t, u, v, ng, tmin, hit.t, ro, rd, v0, v1, v2)) {
-            hit.t = t;
-            hit.u = u;
-            hit.v = v;
-            hit.ng = ng;
-            hit.tri = ti;
-            if (kAny) return true;
-        }
+        if (replay_leaf<kAny>(curr, hit, tris, ro, rd, tmin)) return true;
     } else {
         if (kCount) ++nv;
-        const NodeView nd = load_node<true>(nodes, curr);
-        const float2 rl = slab(ro, inv, nd.lo0, nd.hi0, tmin, hit.t);
-        const float2 rr = slab(ro, inv, nd.lo1, nd.hi1, tmin, hit.t);
-        const bool hitL = rl.x <= rl.y, hitR = rr.x <= rr.y;
-        if (hitL && hitR) {
-            const bool swap = rr.x < rl.x;
-            const uint32_t nearN = swap ? nd.c1 : nd.c0, farN = swap ? nd.c0 : nd.c1;
-            if (depth == kDepth) {  // full: continue as the stack-free walk
-                depth = -1;
-                prev = curr;
-                curr = nearN;
-                return false;
-            }
-            if constexpr (kAny)
-                stack[depth * stride] = farN;
-            else
-                stack[depth * stride] = make_uint2(farN, __float_as_uint(swap ? rl.x : rr.x));
-            ++depth;
-            curr = nearN;
-            return false;
-        }
-        if (hitL || hitR) {
-            curr = hitL ? nd.c0 : nd.c1;
-            return false;
-        }
+        if (replay_node<kAny, kDepth>(curr, prev, depth, stack, stride, hit.t, nodes, ro, inv, tmin)) return false;
     }
-    if constexpr (kAny) {
-        if (depth == 0) return true;
-        curr = stack[--depth * stride];
-        return false;
-    } else {
-        while (depth > 0) {
-            const uint2 e = stack[--depth * stride];
-            if (__uint_as_float(e.y) <= hit.t) {
-                curr = e.x;
-                return false;
-            }
-        }
-        return true;
-    }
+    return replay_pop<kAny>(curr, depth, stack, stride, hit.t);
 }
 
 // The replay walk over leaf-ordered triangles: mlbvh_qtri records (48 bytes,

@@ -15,6 +15,8 @@
 // stored; Vicini et al., "Path Replay Backpropagation", 2021): with c_d the
 // radiance collected at vertex d, dL/da(t_j) = (sum_{d>j} c_d) / a(t_j), and
 // grad[t_j] += dLoss/dI_p / spp * that, scattered with atomic adds.
+#include <algorithm>
+
 #include "capi_internal.h"
 #include "../../include/mlbvh_device.cuh"
 
@@ -22,100 +24,28 @@ namespace mlbvh {
 
 namespace {
 
-// Threads per CTA: one pixel's warp (measured forward / adjoint ms: 22.6 / 18.0
-// against 22.6 / 18.3 for 64 and 22.7 / 19.1 for 128, where a CTA holds its
-// slot until its slowest pixel is done); compiled for 768 threads per SM (80
-// registers). Build-time override for sweeps: -DMLBVH_DIFF_THREADS.
-#ifndef MLBVH_DIFF_THREADS
-#define MLBVH_DIFF_THREADS 32
-#endif
-constexpr int kDiffThreads = MLBVH_DIFF_THREADS;
+// What follows was swept on the differentiation workload (heightfield, 512x512,
+// 64 samples, 3 bounces; forward / adjoint ms, start 23.1 / 24.6). Warps per SM
+// the kernels are compiled for: 24 19.2 / 19.5, 28 17.9 / 18.2, 32 (64
+// registers) 17.2 / 17.2, 40 20.4 / 19.4 (spills). Node visits per round and
+// lane: 3 16.9 / 17.5, 4 16.6 / 17.1, 5 16.7 / 16.9, 6 16.8 / 17.1, 8 17.4 /
+// 17.4; nodes and leaves in one step, whichever a lane is at: 21.5 / 21.6 (a
+// round then pays for both in nearly every step). Lanes that wait before the
+// next rays are set up: 8 17.3 / 17.4, 10 16.6 / 17.0, 12 16.6 / 17.1, 16 17.4 /
+// 17.4. Leaf tests held back until 8 lanes wait: no gain, 16 lanes: 19.3.
+constexpr int kDiffThreads = 64;
+constexpr int kDiffWarps = 32;
+constexpr int kDiffSteps = 4;
+constexpr int kDiffService = 10;
 constexpr int kMaxBounces = 8;
-// Lanes per pixel: one warp per pixel, lane l tracing samples l, l + 32, ...
-// in order; the render adds the lanes' partial sums as a pairwise tree in lane
-// order ((p0 + p1) + (p2 + p3)) + ... . Measured on the differentiation
-// workload (forward / adjoint ms): one thread per pixel 35.3 / 32.3 (2.3 waves
-// of long CTAs, the last on a third of the SMs), 2 lanes 30.1 / 27.1, 4 lanes
-// 26.5 / 23.3, 8 lanes 24.4 / 21.0, 16 lanes 23.2 / 19.6, 32 lanes 22.7 / 18.3:
-// a pixel's samples start from nearby rays, so its warp walks the same nodes.
-// (Build-time override for sweeps: -DMLBVH_DIFF_LANES=2, 4, 8 or 16.)
-#ifndef MLBVH_DIFF_LANES
-#define MLBVH_DIFF_LANES 32
-#endif
-constexpr int kLanesPerPixel = MLBVH_DIFF_LANES;
-static_assert(kDiffThreads % kLanesPerPixel == 0, "a pixel's lanes share a warp");
-constexpr int kDiffStack = 16;  // replay-walk stack entries per thread (shared memory)
-
-// intersect_stackfree's closest hit (minimum_lbvh.h:981-1061) through the
-// replay walk (stackfree_replay_step): the same Hit record, ties included,
-// with every internal node loaded once. `stack` is this thread's column of a
-// kDiffStack x kDiffThreads shared-memory array.
-__device__ __forceinline__ void trace_closest(HitRecord& hit, const mlbvh_internal_node* __restrict__ nodes,
-                                              const float* __restrict__ tris, uint32_t root, f3 ro, f3 rd,
-                                              uint2* stack)
-{
-    const f3 inv = inv_rd(rd);
-    uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0;
-    int depth = 0;
-    for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps)
-        if (stackfree_replay_step<false, false, kDiffStack>(curr, prev, depth, stack, kDiffThreads, hit, nodes, tris,
-                                                             ro, rd, inv, 0.0f, nv, nt))
-            break;
-}
+constexpr int kDiffStack = 16;       // replay-walk stack entries per lane (shared memory)
+constexpr uint32_t kUnit = 64;       // samples per unit of the render's ordered sums; two units are open at a time
+constexpr uint32_t kWarpSamples = 512;  // samples a warp takes where the image has enough pixels
 
 struct PathVertex {
     uint32_t tri;
     float collected;  // throughput * emission at this vertex
 };
-
-// Traces the path of sample s of pixel (xi, yi). kStore: fills v (at most
-// bounces + 1 vertices) and returns the vertex count; otherwise adds the
-// collected radiance, vertex by vertex in path order, to *L (the same sum the
-// forward render forms from v) and keeps no vertices.
-template <bool kStore>
-__device__ __forceinline__ int trace_path(PathVertex* v, float* L, int bounces, uint32_t s, int xi, int yi, int w, int h,
-                                          const Camera& cam, uint32_t root, const mlbvh_internal_node* __restrict__ nodes,
-                                          const float* __restrict__ tris, const float* __restrict__ albedo,
-                                          const float* __restrict__ emission, uint2* stack)
-{
-    const float2 jitter = sobol2d(s, (uint32_t)xi, (uint32_t)yi, 0u);
-    f3 ro, rd;
-    shoot(cam, ((float)xi + jitter.x) / (float)w, ((float)yi + jitter.y) / (float)h, ro, rd);
-    HitRecord hit;
-    hit.t = kFltMax;
-    hit.tri = 0xFFFFFFFFu;
-    trace_closest(hit, nodes, tris, root, ro, rd, stack);
-    if (hit.t == kFltMax) return 0;
-    float throughput = 1.0f;
-    int count = 0;
-    for (int d = 0; d <= bounces; ++d) {
-        const uint32_t t = hit.tri;
-        const float collected = throughput * __ldg(emission + t);
-        if (kStore) {
-            v[count].tri = t;
-            v[count].collected = collected;
-        } else {
-            *L += collected;
-        }
-        ++count;
-        if (d == bounces) break;
-        const f3 p = ro + rd * hit.t;
-        f3 n = normalize(hit.ng);
-        if (0.0f < dot(n, rd)) n = -n;
-        f3 xaxis, zaxis;
-        onb(n, xaxis, zaxis);
-        const float2 r = sobol2d(s, (uint32_t)xi, (uint32_t)yi, (uint32_t)(1 + d));
-        const f3 dl = sample_hemisphere(r.x, r.y);
-        ro = p + n * 0.0001f;
-        rd = xaxis * dl.x + zaxis * dl.z + n * dl.y;
-        throughput = throughput * __ldg(albedo + t);
-        hit.t = kFltMax;
-        hit.tri = 0xFFFFFFFFu;
-        trace_closest(hit, nodes, tris, root, ro, rd, stack);
-        if (hit.t == kFltMax) break;
-    }
-    return count;
-}
 
 __device__ __forceinline__ Camera camera_of(const mlbvh_ray_generator& g)
 {
@@ -126,65 +56,232 @@ __device__ __forceinline__ Camera camera_of(const mlbvh_ray_generator& g)
     return c;
 }
 
-__global__ void __launch_bounds__(kDiffThreads, 768 / kDiffThreads)
-    k_pt_diff_render(float* __restrict__ image, int w, int h, int spp, int bounces, mlbvh_ray_generator gen,
-                     const mlbvh_node_index* __restrict__ rootPtr, const mlbvh_internal_node* __restrict__ nodes,
-                     const float* __restrict__ tris, const float* __restrict__ albedo,
-                     const float* __restrict__ emission)
+struct DiffScene {
+    int w, h, spp, bounces;
+    uint32_t warpPixels;  // consecutive pixels per warp
+    mlbvh_ray_generator gen;
+    const mlbvh_node_index* rootPtr;
+    const mlbvh_internal_node* nodes;
+    const float* tris;
+    const float* albedo;
+    const float* emission;
+};
+
+// Both kernels: a warp traces the samples of `warpPixels` consecutive pixels,
+// numbered pixel by pixel. Every lane works on a path of its own: it walks
+// its ray (intersect_stackfree's closest hit, minimum_lbvh.h:981-1061, through
+// the replay walk), and when the ray is done it waits until kDiffService lanes
+// do (or as many as still walk); those lanes then shade together, go on with their
+// paths' next rays or take the next samples. So a lane whose path ends early
+// takes another instead of idling until the warp's longest path is done (with a
+// pixel per warp 5.6 of 32 threads were active per instruction, now 15). Bound:
+// issue (70 %) and the L1's data stage (76 %).
+//
+// kAdjoint: the path's vertices are kept and the gradient is scattered when the
+// path ends. Otherwise the pixel's radiance is summed in a fixed order,
+// whichever lane traced which sample: lane l adds the samples l, l + 32, ... of
+// the pixel in turn, and the lanes' sums are added as a pairwise tree in lane
+// order, ((p0 + p1) + (p2 + p3)) + ...; the radiances of two units of 64
+// samples are kept in shared memory until the older unit is complete.
+template <bool kAdjoint>
+__device__ __forceinline__ void trace_pixels(const DiffScene& sc, float* __restrict__ image,
+                                             float* __restrict__ grad, const float* __restrict__ gradImage)
 {
     __shared__ uint2 s_stack[kDiffStack][kDiffThreads];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int p = t / kLanesPerPixel, lane = t % kLanesPerPixel;
-    const bool valid = p < w * h;  // every lane takes part in the shuffles below
-    float sum = 0.0f;
-    if (valid) {
-        const int xi = p % w, yi = p / w;
-        const Camera cam = camera_of(gen);
-        const uint32_t root = __ldg(rootPtr);
-        for (int s = lane; s < spp; s += kLanesPerPixel) {
-            float L = 0.0f;
-            trace_path<false>(nullptr, &L, bounces, (uint32_t)s, xi, yi, w, h, cam, root, nodes, tris, albedo,
-                              emission, &s_stack[0][threadIdx.x]);
-            sum += L;
-        }
-    }
-    // the pairwise tree in lane order: after step o every lane holds the sum of
-    // its aligned group of 2o lanes, the same bits on each (a + b == b + a)
+    __shared__ float s_radiance[kAdjoint ? 1 : kDiffThreads / 32][kAdjoint ? 1 : 2 * kUnit];
+    uint2* const stack = &s_stack[0][threadIdx.x];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t pixels = (uint32_t)(sc.w * sc.h), spp = (uint32_t)sc.spp;
+    const uint32_t p0 = (blockIdx.x * (kDiffThreads / 32) + warp) * sc.warpPixels;
+    if (p0 >= pixels) return;
+    const uint32_t total = min(sc.warpPixels, pixels - p0) * spp;
+    const Camera cam = camera_of(sc.gen);
+    const uint32_t root = __ldg(sc.rootPtr);
+    float* const radiance = kAdjoint ? nullptr : s_radiance[kAdjoint ? 0 : warp];
+
+    uint32_t next = 0;         // warp-uniform: samples handed out
+    uint32_t retired = 0;      // warp-uniform (render): samples summed, in whole units
+    uint32_t left0 = kUnit, left1 = kUnit;  // warp-uniform (render): unfinished samples of the open even and odd unit
+    float partial = 0.0f;      // render: this lane's sum of the pixel being retired
+    // the lane's path: the segment in flight (-1: no path), its sample and state
+    int d = -1;
+    bool walking = false;
+    uint32_t sample = 0, s = 0, xi = 0, yi = 0;
+    float throughput = 1.0f, L = 0.0f, g = 0.0f;
+    PathVertex v[kAdjoint ? kMaxBounces + 1 : 1];
+    f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
+    HitRecord hit;
+    hit.t = kFltMax;
+    hit.tri = 0;
+    hit.ng = ro;
+    uint32_t curr = 0, prev = 0, steps = 0;
+    int depth = 0;
+    for (;;) {
+        const uint32_t limit = kAdjoint ? total : min(total, retired + 2 * kUnit);
+        const int walkers = __popc(__ballot_sync(0xffffffffu, walking));
+        const int waiting = __popc(__ballot_sync(0xffffffffu, !walking && (d >= 0 || next < limit)));
+        if (walkers == 0 && waiting == 0) break;
+        if (waiting >= min(kDiffService, max(walkers, 1))) {
+            // ---- shade the hits
+            bool start = false, ended = false;
+            f3 p = ro, n = ro;
+            if (!walking && d >= 0) {
+                if (hit.t == kFltMax) {
+                    ended = true;
+                } else {
+                    const uint32_t t = hit.tri;
+                    const float collected = throughput * __ldg(sc.emission + t);
+                    if (kAdjoint) {
+                        v[d].tri = t;
+                        v[d].collected = collected;
+                    } else {
+                        L += collected;
+                    }
+                    if (d++ == sc.bounces) {
+                        ended = true;
+                    } else {
+                        p = ro + rd * hit.t;
+                        n = normalize(hit.ng);
+                        if (0.0f < dot(n, rd)) n = -n;
+                        throughput = throughput * __ldg(sc.albedo + t);
+                        start = true;
+                    }
+                }
+            }
+            if (kAdjoint) {
+                if (ended) {
+                    // suffix sums of the collected radiance: the part of L that depends on
+                    // the albedo of vertex j is everything collected after it
+                    float after = 0.0f;
+                    for (int j = d - 1; j >= 0; --j) {
+                        if (j < sc.bounces && after != 0.0f) {
+                            const uint32_t tj = v[j].tri;
+                            atomicAdd(grad + tj, g * after / __ldg(sc.albedo + tj));
+                        }
+                        after += v[j].collected;
+                    }
+                }
+            } else {
+                if (ended) radiance[sample % (2 * kUnit)] = L;
+                left0 -= __popc(__ballot_sync(0xffffffffu, ended && !(sample & kUnit)));
+                left1 -= __popc(__ballot_sync(0xffffffffu, ended && (sample & kUnit)));
+                __syncwarp();
+                while (retired < next && ((retired & kUnit) ? left1 : left0) == kUnit - min(kUnit, total - retired)) {
+                    // a unit is complete: add its samples to their pixels
+                    const uint32_t unitEnd = retired + min(kUnit, total - retired);
+                    for (uint32_t i = retired; i < unitEnd;) {
+                        const uint32_t pix = i / spp, s0 = i - pix * spp, end = min(unitEnd, (pix + 1) * spp);
+                        for (uint32_t k = i + ((lane - s0) & 31u); k < end; k += 32)
+                            partial += radiance[k % (2 * kUnit)];
+                        if (end == (pix + 1) * spp) {
+                            float sum = partial;
 #pragma unroll
-    for (int o = 1; o < kLanesPerPixel; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (valid && lane == 0) image[p] = sum / (float)spp;
+                            for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                            if (lane == 0) image[p0 + pix] = sum / (float)spp;
+                            partial = 0.0f;
+                        }
+                        i = end;
+                    }
+                    if (retired & kUnit)
+                        left1 = kUnit;
+                    else
+                        left0 = kUnit;
+                    retired += kUnit;
+                    __syncwarp();
+                }
+            }
+            if (ended) d = -1;
+            // ---- lanes without a path take the next samples
+            const uint32_t end = kAdjoint ? total : min(total, retired + 2 * kUnit);
+            const uint32_t idle = __ballot_sync(0xffffffffu, d < 0);
+            const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+            if (d < 0 && next < end && rank < end - next) {
+                sample = next + rank;
+                const uint32_t pix = sample / spp, pixel = p0 + pix;
+                s = sample - pix * spp;
+                xi = pixel % (uint32_t)sc.w;
+                yi = pixel / (uint32_t)sc.w;
+                throughput = 1.0f;
+                L = 0.0f;
+                d = 0;
+                start = true;
+                if (kAdjoint) {
+                    g = __ldg(gradImage + pixel) / (float)sc.spp;
+                    if (g == 0.0f) {  // nothing to scatter
+                        d = -1;
+                        start = false;
+                    }
+                }
+            }
+            next = min(next + (uint32_t)__popc(idle), max(end, next));
+            // ---- the next rays
+            if (start) {
+                const float2 r = sobol2d(s, xi, yi, (uint32_t)d);
+                if (d == 0) {
+                    shoot(cam, ((float)xi + r.x) / (float)sc.w, ((float)yi + r.y) / (float)sc.h, ro, rd);
+                } else {
+                    f3 xaxis, zaxis;
+                    onb(n, xaxis, zaxis);
+                    const f3 dl = sample_hemisphere(r.x, r.y);
+                    ro = p + n * 0.0001f;
+                    rd = xaxis * dl.x + zaxis * dl.z + n * dl.y;
+                }
+                inv = inv_rd(rd);
+                hit.t = kFltMax;
+                hit.tri = 0xFFFFFFFFu;
+                curr = root;
+                prev = kInvalid;
+                depth = 0;
+                steps = 0;
+                walking = true;
+            }
+        }
+        // ---- node visits, then the leaf tests
+#pragma unroll
+        for (int rep = 0; rep < kDiffSteps; ++rep)
+            if (walking && !(curr & kLeafBit) && depth >= 0)
+                if (!replay_node<false, kDiffStack>(curr, prev, depth, stack, kDiffThreads, hit.t, sc.nodes, ro, inv,
+                                                    0.0f))
+                    walking = !replay_pop<false>(curr, depth, stack, kDiffThreads, hit.t);
+        if (walking && ((curr & kLeafBit) || depth < 0)) {
+            uint32_t nv = 0, nt = 0;
+            walking = !stackfree_replay_step<false, false, kDiffStack>(curr, prev, depth, stack, kDiffThreads, hit,
+                                                                       sc.nodes, sc.tris, ro, rd, inv, 0.0f, nv, nt);
+        }
+        steps += kDiffSteps + 1;
+        if (steps >= kMaxTraversalSteps) walking = false;
+    }
 }
 
-__global__ void __launch_bounds__(kDiffThreads, 768 / kDiffThreads)
-    k_pt_diff_adjoint(float* __restrict__ grad, const float* __restrict__ gradImage, int w, int h, int spp,
-                      int bounces, mlbvh_ray_generator gen, const mlbvh_node_index* __restrict__ rootPtr,
-                      const mlbvh_internal_node* __restrict__ nodes, const float* __restrict__ tris,
-                      const float* __restrict__ albedo, const float* __restrict__ emission)
+__global__ void __launch_bounds__(kDiffThreads, kDiffWarps * 32 / kDiffThreads)
+    k_pt_diff_render(float* __restrict__ image, DiffScene sc)
 {
-    __shared__ uint2 s_stack[kDiffStack][kDiffThreads];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int p = t / kLanesPerPixel, lane = t % kLanesPerPixel;
-    if (p >= w * h) return;
-    const float g = __ldg(gradImage + p) / (float)spp;
-    if (g == 0.0f) return;
-    const int xi = p % w, yi = p / w;
-    const Camera cam = camera_of(gen);
-    const uint32_t root = __ldg(rootPtr);
-    PathVertex v[kMaxBounces + 1];
-    for (int s = lane; s < spp; s += kLanesPerPixel) {
-        const int n = trace_path<true>(v, nullptr, bounces, (uint32_t)s, xi, yi, w, h, cam, root, nodes, tris, albedo,
-                                       emission, &s_stack[0][threadIdx.x]);
-        // suffix sums of the collected radiance: the part of L that depends on
-        // the albedo of vertex j is everything collected after it
-        float after = 0.0f;
-        for (int j = n - 1; j >= 0; --j) {
-            if (j < bounces && after != 0.0f) {
-                const uint32_t tj = v[j].tri;
-                atomicAdd(grad + tj, g * after / __ldg(albedo + tj));
-            }
-            after += v[j].collected;
-        }
-    }
+    trace_pixels<false>(sc, image, nullptr, nullptr);
+}
+
+__global__ void __launch_bounds__(kDiffThreads, kDiffWarps * 32 / kDiffThreads)
+    k_pt_diff_adjoint(float* __restrict__ grad, const float* __restrict__ gradImage, DiffScene sc)
+{
+    trace_pixels<true>(sc, nullptr, grad, gradImage);
+}
+
+// Pixels per warp: kWarpSamples samples at most, two rounds of resident warps
+// where that leaves a warp 32 samples, else 32 samples (a warp's lanes share
+// its instructions) as long as 16 warps per SM remain: few samples finish
+// soonest spread out. The samples of a warp stay below 2^31.
+uint32_t warp_pixels(int w, int h, int spp)
+{
+    const unsigned long long samples = (unsigned long long)w * h * (unsigned long long)spp;
+    const uint32_t sms = (uint32_t)device_sm_count();
+    unsigned long long k = std::min<unsigned long long>(samples / (2u * kDiffWarps * sms), kWarpSamples);
+    if (k < 32) k = std::min<unsigned long long>(32, samples / (16u * sms));
+    return (uint32_t)std::max<unsigned long long>(1, (k + (unsigned)spp - 1) / (unsigned)spp);
+}
+uint32_t diff_blocks(const DiffScene& sc)
+{
+    const uint32_t pixels = (uint32_t)sc.w * (uint32_t)sc.h;
+    const uint32_t perBlock = sc.warpPixels * (kDiffThreads / 32);
+    return (pixels + perBlock - 1) / perBlock;
 }
 
 mlbvh_status check_diff_args(int w, int h, int spp, int bounces, const void* a, const void* b, const void* c,
@@ -208,10 +305,10 @@ mlbvh_status pt_diff_render(float* dImage, int w, int h, int spp, int bounces, c
 {
     if (mlbvh_status s = check_diff_args(w, h, spp, bounces, dImage, dRoot, dTris, dAlbedo, dEmission)) return s;
     if (!aligned32(dNodes)) return fail(MLBVH_ERR_INVALID_ARG, "device pointers must be 16-byte aligned");
-    const long long threads = (long long)w * h * kLanesPerPixel;
-    if (threads >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
-    k_pt_diff_render<<<(unsigned)((threads + kDiffThreads - 1) / kDiffThreads), kDiffThreads, 0, stream>>>(
-        dImage, w, h, spp, bounces, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo, dEmission);
+    if ((long long)w * h * 32 >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
+    const DiffScene sc{w, h, spp, bounces, warp_pixels(w, h, spp), cam, dRoot, dNodes,
+                       reinterpret_cast<const float*>(dTris), dAlbedo, dEmission};
+    k_pt_diff_render<<<diff_blocks(sc), kDiffThreads, 0, stream>>>(dImage, sc);
     MLBVH_CHECK_LAUNCH("k_pt_diff_render");
     return MLBVH_OK;
 }
@@ -224,11 +321,10 @@ mlbvh_status pt_diff_adjoint(float* dGrad, const float* dGradImage, int w, int h
     if (mlbvh_status s = check_diff_args(w, h, spp, bounces, dGrad, dRoot, dTris, dAlbedo, dEmission)) return s;
     if (!dGradImage || !aligned16(dGradImage) || !aligned32(dNodes))
         return fail(MLBVH_ERR_INVALID_ARG, "null or misaligned pointer");
-    const long long threads = (long long)w * h * kLanesPerPixel;
-    if (threads >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
-    k_pt_diff_adjoint<<<(unsigned)((threads + kDiffThreads - 1) / kDiffThreads), kDiffThreads, 0, stream>>>(
-        dGrad, dGradImage, w, h, spp, bounces, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo,
-        dEmission);
+    if ((long long)w * h * 32 >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
+    const DiffScene sc{w, h, spp, bounces, warp_pixels(w, h, spp), cam, dRoot, dNodes,
+                       reinterpret_cast<const float*>(dTris), dAlbedo, dEmission};
+    k_pt_diff_adjoint<<<diff_blocks(sc), kDiffThreads, 0, stream>>>(dGrad, dGradImage, sc);
     MLBVH_CHECK_LAUNCH("k_pt_diff_adjoint");
     return MLBVH_OK;
 }
