@@ -487,6 +487,26 @@ __device__ __forceinline__ bool stackfree_replay_step_lo(uint32_t& curr, uint32_
     }
 }
 
+// A whole walk of a thread's ray in phases: up to kNodes node visits, then one
+// leaf test. A warp's lanes are at nodes far more often than at leaves, but
+// with one step of either kind at a time nearly every step of the warp has
+// some lane at a leaf and so pays for both; in phases a round pays for kNodes
+// visits and one test. `step` makes one step (curr, depth: its state; a
+// negative depth is a walk that handles nodes and leaves alike) and returns
+// true when the walk is over. Each lane's own steps are those of the plain loop.
+template <int kNodes, class Step>
+__device__ __forceinline__ void walk_phases(const uint32_t& curr, const int& depth, Step step)
+{
+    bool done = false;
+    for (uint32_t steps = 0; steps < kMaxTraversalSteps; steps += kNodes + 1) {
+#pragma unroll
+        for (int k = 0; k < kNodes; ++k)
+            if (!done && !(curr & kLeafBit) && depth >= 0) done = step();
+        if (!done && ((curr & kLeafBit) || depth < 0)) done = step();
+        if (done) return;
+    }
+}
+
 template <bool kAny, bool kCount = false, bool kWide = false>
 __device__ __forceinline__ void trace_stackfree(HitRecord& hit, const mlbvh_internal_node* __restrict__ nodes,
                                                 const float* __restrict__ tris, uint32_t root, f3 ro, f3 rd,

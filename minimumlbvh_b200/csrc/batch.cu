@@ -388,6 +388,10 @@ struct MeshTrees {
 // mlbvh_trace writes them; ray i of the batch belongs to the mesh m with
 // rayOff[m] <= i < rayOff[m+1].
 constexpr int kBatchReplayDepth = 16;  // stack entries per lane of the replay walk
+// Node visits per round, each followed by one leaf test (256 meshes, 9M rays,
+// trace alone): one step of either kind per round 1,313 us; 1 1,366, 2 1,174,
+// 3 1,111, 4 1,092, 5 1,085, 6 1,081.
+constexpr int kBatchNodeSteps = 5;
 
 template <bool kAny, bool kReplay>
 __global__ void __launch_bounds__(512)
@@ -469,18 +473,24 @@ __global__ void __launch_bounds__(512)
             continue;
         }
         if (live) {
-            // an index outside the mesh's tree (possible only in a corrupt tree) ends the walk
-            const bool inTree = (curr & kLeafBit) ? (curr & ~kLeafBit) < leaves : curr + 1 < leaves;
-            bool done = !inTree;
-            if (!done) {
+            auto step = [&] {
+                // an index outside the mesh's tree (possible only in a corrupt tree) ends the walk
+                if ((curr & kLeafBit) ? (curr & ~kLeafBit) >= leaves : curr + 1 >= leaves) return true;
                 if constexpr (kReplay)
-                    done = stackfree_replay_step<kAny, false, kBatchReplayDepth>(curr, prev, depth, stack, blockDim.x,
+                    return stackfree_replay_step<kAny, false, kBatchReplayDepth>(curr, prev, depth, stack, blockDim.x,
                                                                                   hit, mn, mt, ro, rd, inv, tmin, nv,
                                                                                   nt);
                 else
-                    done = stackfree_step<kAny, false, true>(curr, prev, hit, mn, mt, ro, rd, inv, tmin, nv, nt);
-            }
-            if (done || ++steps >= kMaxTraversalSteps) {
+                    return stackfree_step<kAny, false, true>(curr, prev, hit, mn, mt, ro, rd, inv, tmin, nv, nt);
+            };
+            // node visits, then a leaf test (see walk_phases)
+            bool done = false;
+#pragma unroll
+            for (int k = 0; k < kBatchNodeSteps; ++k)
+                if (!done && !(curr & kLeafBit) && depth >= 0) done = step();
+            if (!done && ((curr & kLeafBit) || depth < 0)) done = step();
+            steps += kBatchNodeSteps + 1;
+            if (done || steps >= kMaxTraversalSteps) {
                 hits[2 * (size_t)ray] = make_float4(hit.t, 0.0f, hit.u, hit.v);
                 hits[2 * (size_t)ray + 1] = make_float4(hit.ng.x, hit.ng.y, hit.ng.z, __uint_as_float(hit.tri));
                 live = false;

@@ -22,37 +22,50 @@ namespace {
 constexpr int kTileW = 16, kTileH = 8;  // 128-thread pixel tile: 4 warps of 8 x 4 pixels
 constexpr int kAoThreads = 128;
 
-// Build-time overrides for tuning sweeps (-DMLBVH_AO_START_BATCH=...).
-#ifndef MLBVH_AO_START_BATCH
-#define MLBVH_AO_START_BATCH 8
-#endif
+// Build-time overrides for tuning sweeps (-DMLBVH_AO_START_BATCH=...). Swept on
+// whole frames (heightfield 512x512, 16 rays per hit / 4M-triangle soup
+// 1920x1080, 64 rays; us). Node visits per leaf test: binary replay 1 1,322 /
+// 14,479, 2 1,184 / 12,425, 3 1,144 / 11,664, 4 1,139 / 11,404, 6 1,167 /
+// 11,211; 4-wide 2 1,110 / 11,920, 3 1,105 / 11,638, 4 1,128 / 11,569;
+// quantised 4-wide 2 1,144 / 11,332, 3 1,163 / 10,993, 4 1,199 / 10,998;
+// quantised binary 3 1,295 / 13,088, 4 1,281 / 12,565, 6 1,352 / 12,628. (One
+// step of either kind at a time, at its best step count: 1,310 / 14,660, 1,170 /
+// 12,808, 1,189 / 12,888, 1,459 / 16,719.)
 #ifndef MLBVH_AO_STEPS_PER_ROUND
-#define MLBVH_AO_STEPS_PER_ROUND 3
+#define MLBVH_AO_STEPS_PER_ROUND 4
 #endif
 #ifndef MLBVH_AO_WIDE_STEPS_PER_ROUND
-#define MLBVH_AO_WIDE_STEPS_PER_ROUND 2
+#define MLBVH_AO_WIDE_STEPS_PER_ROUND 3
 #endif
 #ifndef MLBVH_AO_QWIDE_STEPS_PER_ROUND
-#define MLBVH_AO_QWIDE_STEPS_PER_ROUND 1
+#define MLBVH_AO_QWIDE_STEPS_PER_ROUND 3
 #endif
+// Free lanes that wait before new rays are set up: 4, 6, 8, 12 on the soup:
+// 4-wide 12,330, 11,936, 11,650, 11,343; binary replay 11,929, 11,600, 11,421,
+// 11,394; quantised 4-wide 11,124, 10,973, 10,994, 11,310; quantised binary
+// 12,696, 12,509, 12,576, 12,908.
+#ifndef MLBVH_AO_START_BATCH
+#define MLBVH_AO_START_BATCH 12
+#endif
+#ifndef MLBVH_AO_WIDE_START_BATCH
+#define MLBVH_AO_WIDE_START_BATCH 12
+#endif
+#ifndef MLBVH_AO_QUANT_START_BATCH
+#define MLBVH_AO_QUANT_START_BATCH 8
+#endif
+// Resident CTAs per SM: 8 (64 registers) against 9 and 10 on the soup: 4-wide
+// 11,650, 11,906, 12,441; quantised 4-wide 10,994, 11,091, 11,071; binary
+// replay 11,421, 11,474, 11,273. Quantised binary: 9 12,576, 8 12,955, 10 13,036.
 #ifndef MLBVH_AO_MIN_BLOCKS
 #define MLBVH_AO_MIN_BLOCKS 8
 #endif
 #ifndef MLBVH_AO_QUANT_MIN_BLOCKS
 #define MLBVH_AO_QUANT_MIN_BLOCKS 9
 #endif
-// resident CTAs per SM of the AO kernel over quantised 4-wide slots (swept: 9
-// and 10, at 56 and 48 registers, ran 3 and 4 % slower than 8 at 63)
 #ifndef MLBVH_AO_QWIDE_MIN_BLOCKS
 #define MLBVH_AO_QWIDE_MIN_BLOCKS 8
 #endif
-// the stack-free walk's own (swept: 4 steps and a batch of 16 lanes beat 3 and
-// 8 by 1.7 %; a batch of 24 loses 7 %)
-// the wide trees' refill batch (swept 4-16: 8 is best for the quantised slots,
-// within 1 % of the best for the FP32 ones)
-#ifndef MLBVH_AO_WIDE_START_BATCH
-#define MLBVH_AO_WIDE_START_BATCH 8
-#endif
+// The stack-free walk's own (its counting variant only).
 #ifndef MLBVH_AO_PLAIN_STEPS_PER_ROUND
 #define MLBVH_AO_PLAIN_STEPS_PER_ROUND 4
 #endif
@@ -195,6 +208,7 @@ __device__ __forceinline__ bool box_meets(f3 lo, f3 hi, const AoBall& b)
 // the replay walk. Primary rays of the replay forms take the closest-hit
 // replay walk (pstack: 16 entries per thread in shared memory).
 constexpr int kReplayDepth = 16;
+constexpr int kPrimarySteps = 3;  // node visits per leaf test of the one-ray-per-thread walks (walk_phases)
 template <int kWalk>
 struct PlainTreeT {
     const mlbvh_internal_node* nodes;
@@ -259,8 +273,9 @@ struct PlainTreeT {
             const f3 inv = inv_rd(rd);
             uint32_t curr = c.root, prev = kInvalid;
             int depth = 0;
-            for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps)
-                if (walk<false, kCount>(curr, prev, depth, pstack, stride, hit, ro, rd, inv, n)) break;
+            walk_phases<kPrimarySteps>(curr, depth, [&] {
+                return walk<false, kCount>(curr, prev, depth, pstack, stride, hit, ro, rd, inv, n);
+            });
         }
     }
     template <bool kAny, bool kCount>
@@ -297,10 +312,11 @@ struct QuantTree {
         const QParams qp{c.eb, c.status, c.status == 0u && qwide_ray_fits(ro, inv)};
         uint32_t curr = c.root, prev = kInvalid;
         int depth = 0;
-        for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps)
-            if (quantised_replay_step<false, kCount, kStack>(curr, prev, depth, pstack, stride, hit, qnodes, parents,
-                                                            qtris, qp, ro, rd, inv, 0.0f, n.visits, n.tests, n.ups))
-                break;
+        walk_phases<kPrimarySteps>(curr, depth, [&] {
+            return quantised_replay_step<false, kCount, kStack>(curr, prev, depth, pstack, stride, hit, qnodes, parents,
+                                                                qtris, qp, ro, rd, inv, 0.0f, n.visits, n.tests,
+                                                                n.ups);
+        });
     }
     // the replay walk: the stack-free walk's leaf order with a stack of
     // kStack pending far children per lane (shared memory) instead of revisits;
@@ -308,6 +324,7 @@ struct QuantTree {
     static constexpr int kStack = 16;
     static constexpr int kPrimaryStack = kStack;
     static constexpr int kMinBlocks = MLBVH_AO_QUANT_MIN_BLOCKS;
+    static constexpr int kStartBatch = MLBVH_AO_QUANT_START_BATCH;
     __device__ __forceinline__ uint32_t ball_start(const Ctx& c, const AoBall& b) const
     {
         if (c.status & 2u) return c.root;  // every box passes: no box bounds the ball
@@ -354,7 +371,7 @@ struct WideTreeT {
     static constexpr int kStack = kWideDepth;
     static constexpr int kPrimaryStack = PlainReplayLeafTree::kStack;
     static constexpr int kSteps = kQuant ? MLBVH_AO_QWIDE_STEPS_PER_ROUND : MLBVH_AO_WIDE_STEPS_PER_ROUND;
-    static constexpr int kStartBatch = MLBVH_AO_WIDE_START_BATCH;
+    static constexpr int kStartBatch = kQuant ? MLBVH_AO_QUANT_START_BATCH : MLBVH_AO_WIDE_START_BATCH;
     static constexpr int kMinBlocks = kQuant ? MLBVH_AO_QWIDE_MIN_BLOCKS : MLBVH_AO_MIN_BLOCKS;
     __device__ __forceinline__ Ctx context() const
     {
@@ -494,18 +511,18 @@ __global__ void __launch_bounds__(kTileW* kTileH)
 // i % nSamples). A warp takes kChunk consecutive items per atomic on the work
 // counter, so its lanes mostly trace samples of the same pixel: rays from one
 // origin share their upper paths, and the warp's node loads coalesce. Each
-// lane traces its own ray one node (or leaf) per loop iteration and takes the
-// next item as soon as it is free, so lanes never wait for the longest ray of
-// their warp. Setting a ray up (Sobol point, hemisphere direction, reciprocal
-// direction) costs about as much as several traversal steps, so free lanes
-// take items once kStartBatch of them are free (or none is busy), and the
-// set-up runs for many lanes at once. An occluded ray adds one to its pixel's
-// count; the lanes of a warp add per pixel with one atomic.
+// lane traces its own ray and takes the next item as soon as it is free, so
+// lanes never wait for the longest ray of their warp. A round is up to
+// StepsOf<Tree> node visits per lane, then one leaf test: with a step of
+// either kind at a time nearly every step of the warp paid for both. Setting a
+// ray up (Sobol point, hemisphere direction, reciprocal direction) costs about
+// as much as several traversal steps, so free lanes take items once
+// kStartBatch of them are free (or none is busy), and the set-up runs for many
+// lanes at once. An occluded ray adds one to its pixel's count; the lanes of a
+// warp add per pixel with one atomic.
 constexpr int kChunk = 64;
 constexpr int kStartBatch = MLBVH_AO_START_BATCH;
-// Traversal steps per lane between two refill checks: a tree's kSteps (the
-// wide tree's steps are about twice as long: 2; its quantised steps longer
-// still: 1, measured 2 % faster than 2), else kStepsPerRound.
+// Node visits per lane and round: a tree's kSteps, else kStepsPerRound.
 constexpr int kStepsPerRound = MLBVH_AO_STEPS_PER_ROUND;
 template <class Tree, class = void>
 struct StepsOf {
@@ -615,19 +632,24 @@ __global__ void __launch_bounds__(kAoThreads, MinBlocksOf<Tree>::value)
             if (exhausted) break;
             continue;
         }
-        // up to StepsOf<Tree> steps per loop iteration: the refill and vote
-        // overhead of an iteration is shared by several steps
+        // a round: node visits, then the leaf tests
         bool occluded = false;
 #pragma unroll
         for (int rep = 0; rep < StepsOf<Tree>::value; ++rep)
-            if (live) {
-                if (tree.template step<true, kCount>(ctx, curr, prev, depth, stack, hit, origin, dir, inv, cnt,
-                                                     fits) ||
-                    ++steps >= kMaxTraversalSteps) {
+            if (live && !(curr & kLeafBit) && depth >= 0) {
+                if (tree.template step<true, kCount>(ctx, curr, prev, depth, stack, hit, origin, dir, inv, cnt, fits)) {
                     live = false;
                     occluded = hit.t != radius;
                 }
             }
+        if (live && ((curr & kLeafBit) || depth < 0)) {
+            if (tree.template step<true, kCount>(ctx, curr, prev, depth, stack, hit, origin, dir, inv, cnt, fits)) {
+                live = false;
+                occluded = hit.t != radius;
+            }
+        }
+        steps += StepsOf<Tree>::value + 1;
+        if (steps >= kMaxTraversalSteps) live = false;
         // one atomic per pixel among the lanes whose ray just ended occluded
         uint32_t pending = __ballot_sync(0xffffffffu, occluded);
         while (pending) {
