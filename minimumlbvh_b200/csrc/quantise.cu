@@ -12,21 +12,16 @@
 // leaf j+1 (node j splits leaves j and j+1).
 #include "capi_internal.h"
 #include "../../include/mlbvh_device.cuh"
+#include "ray_pool.cuh"
 
 namespace mlbvh {
 
 namespace {
 
-constexpr int kQuantiseThreads = 256;
-// Threads per CTA of k_trace_quantised: a CTA holds its slot until its longest
-// ray is done (1M camera / random rays of the 4M soup, replay walk: 128 threads
-// 0.599 / 1.59 ms, 64 0.578 / 1.52, 32 0.604 / 1.57). Build-time override for
-// sweeps: -DMLBVH_QTRACE_THREADS.
-#ifndef MLBVH_QTRACE_THREADS
-#define MLBVH_QTRACE_THREADS 64
-#endif
-constexpr int kTraceThreads = MLBVH_QTRACE_THREADS;
+constexpr int kNodeSteps = 4;  // node visits per leaf test (2: 5 % slower)
+constexpr int kPoolWarps = 32;  // resident warps per SM of the pooled trace kernel (64 registers)
 
+constexpr int kQuantiseThreads = 256;
 __device__ __forceinline__ void leaf_box(const float* __restrict__ tris, uint32_t t, f3& lo, f3& hi)
 {
     f3 v0, v1, v2;
@@ -205,75 +200,81 @@ __global__ void __launch_bounds__(kQuantiseThreads)
     if (c1 & kLeafBit) write_qtri(leafTris, j + 1, tris, c1 & ~kLeafBit);
 }
 
-// One thread per ray. kDepth = 0: the stack-free walk (trace_quantised);
+// The rays of a pool (ray_pool.cuh). kDepth = 0: the stack-free walk (trace_quantised);
 // otherwise the replay walk with a kDepth-entry stack per thread in shared
 // memory (quantised_replay_step), which returns the same Hit records.
 // counts (may be null): per ray, internal-node visits, triangle tests and
-// parent loads at counts[i], counts[n + i], counts[2n + i].
+// parent loads at counts[i], counts[pool.n + i], counts[2n + i].
 template <bool kAny, int kDepth, bool kCount>
-__global__ void __launch_bounds__(kTraceThreads)
+__global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
     k_trace_quantised(const mlbvh_qnode* __restrict__ qnodes, const uint32_t* __restrict__ parents,
                       const mlbvh_qtri* __restrict__ qtris, const mlbvh_qheader* __restrict__ header,
-                      const float4* __restrict__ rays, float4* __restrict__ hits, uint32_t n,
-                      uint32_t* __restrict__ counts)
+                      const float4* __restrict__ rays, float4* __restrict__ hits,
+                      uint32_t* __restrict__ counts, RayPool pool)
 {
-    __shared__ typename ReplayStack<kAny>::Entry s_stack[kDepth > 0 ? kDepth : 1][kTraceThreads];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
-    const f3 ro = mk(a.x, a.y, a.z), rd = mk(b.x, b.y, b.z);
-    HitRecord hit;
-    hit.t = b.w;
-    hit.u = 0.0f;
-    hit.v = 0.0f;
-    hit.ng = mk(0.0f, 0.0f, 0.0f);
-    hit.tri = 0xFFFFFFFFu;
+    __shared__ typename ReplayStack<kAny>::Entry s_stack[kDepth > 0 ? kDepth : 1][kPoolThreads];
     const uint32_t root = __ldg(&header->root);
-    const f3 inv = inv_rd(rd);
-    const QParams qp = qparams(header, ro, inv);
-    uint32_t nv = 0, nt = 0, nu = 0;
-    if (kDepth == 0) {
-        trace_quantised<kAny, kCount>(hit, qnodes, parents, qtris, root, qp, ro, rd, inv, a.w, &nv, &nt, &nu);
-    } else {
-        uint32_t curr = root, prev = kInvalid;
-        int depth = 0;
-        for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps)
-            if (quantised_replay_step<kAny, kCount, kDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                            kTraceThreads, hit, qnodes, parents, qtris, qp, ro, rd,
-                                                            inv, a.w, nv, nt, nu))
-                break;
-    }
-    hits[2 * (size_t)i] = make_float4(hit.t, 0.0f, hit.u, hit.v);
-    hits[2 * (size_t)i + 1] = make_float4(hit.ng.x, hit.ng.y, hit.ng.z, __uint_as_float(hit.tri));
-    if (kCount) {
-        counts[i] = nv;
-        counts[n + i] = nt;
-        counts[2 * (size_t)n + i] = nu;
-    }
+    QParams qp{__ldg(&header->eBase), __ldg(&header->status), false};
+    f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
+    float tmin = 0.0f;
+    HitRecord hit;
+    uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0, nu = 0;
+    int depth = 0;
+    trace_pool<kNodeSteps>(
+        rays, hits, pool, hit, curr,
+        [&](uint32_t, float4 a, float4 b) {
+            ro = mk(a.x, a.y, a.z);
+            rd = mk(b.x, b.y, b.z);
+            inv = inv_rd(rd);
+            tmin = a.w;
+            hit = HitRecord{b.w, 0.0f, 0.0f, mk(0.0f, 0.0f, 0.0f), 0xFFFFFFFFu};
+            qp.fma = qp.status == 0u && qwide_ray_fits(ro, inv);
+            curr = root;
+            prev = kInvalid;
+            depth = 0;
+            if (kCount) nv = nt = nu = 0;
+        },
+        [&] { return depth < 0; },
+        [&] {
+            if constexpr (kDepth == 0)
+                return quantised_step<kAny, kCount>(curr, prev, hit, qnodes, parents, qtris, qp, ro, rd, inv, tmin, nv,
+                                                    nt, nu);
+            else
+                return quantised_replay_step<kAny, kCount, kDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
+                                                                   kPoolThreads, hit, qnodes, parents, qtris, qp, ro,
+                                                                   rd, inv, tmin, nv, nt, nu);
+        },
+        [&](uint32_t i) {
+            if (kCount) {
+                counts[i] = nv;
+                counts[pool.n + i] = nt;
+                counts[2 * (size_t)pool.n + i] = nu;
+            }
+        });
 }
 
 template <bool kAny, int kDepth>
-void launch_trace_quantised(unsigned blocks, cudaStream_t stream, const mlbvh_qnode* q, const uint32_t* p,
+void launch_trace_quantised(cudaStream_t stream, const mlbvh_qnode* q, const uint32_t* p,
                             const mlbvh_qtri* t, const mlbvh_qheader* h, const float4* rays, float4* hits, uint32_t n,
                             uint32_t* counts)
 {
+    const RayPool pool = ray_pool(n, device_sm_count(), kPoolWarps);
     if (counts)
-        k_trace_quantised<kAny, kDepth, true><<<blocks, kTraceThreads, 0, stream>>>(q, p, t, h, rays, hits, n, counts);
+        k_trace_quantised<kAny, kDepth, true><<<pool.ctas, kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, counts, pool);
     else
-        k_trace_quantised<kAny, kDepth, false><<<blocks, kTraceThreads, 0, stream>>>(q, p, t, h, rays, hits, n,
-                                                                                    nullptr);
+        k_trace_quantised<kAny, kDepth, false><<<pool.ctas, kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, nullptr, pool);
 }
 
 template <bool kAny>
-void launch_trace_quantised_depth(int depth, unsigned blocks, cudaStream_t stream, const mlbvh_qnode* q,
+void launch_trace_quantised_depth(int depth, cudaStream_t stream, const mlbvh_qnode* q,
                                   const uint32_t* p, const mlbvh_qtri* t, const mlbvh_qheader* h, const float4* rays,
                                   float4* hits, uint32_t n, uint32_t* counts)
 {
     switch (depth) {
-    case 0: launch_trace_quantised<kAny, 0>(blocks, stream, q, p, t, h, rays, hits, n, counts); break;
-    case 1: launch_trace_quantised<kAny, 1>(blocks, stream, q, p, t, h, rays, hits, n, counts); break;
-    case 4: launch_trace_quantised<kAny, 4>(blocks, stream, q, p, t, h, rays, hits, n, counts); break;
-    default: launch_trace_quantised<kAny, 16>(blocks, stream, q, p, t, h, rays, hits, n, counts); break;
+    case 0: launch_trace_quantised<kAny, 0>(stream, q, p, t, h, rays, hits, n, counts); break;
+    case 1: launch_trace_quantised<kAny, 1>(stream, q, p, t, h, rays, hits, n, counts); break;
+    case 4: launch_trace_quantised<kAny, 4>(stream, q, p, t, h, rays, hits, n, counts); break;
+    default: launch_trace_quantised<kAny, 16>(stream, q, p, t, h, rays, hits, n, counts); break;
     }
 }
 
@@ -326,14 +327,13 @@ mlbvh_status trace_quantised(const mlbvh_qnode* dQNodes, const uint32_t* dQParen
     if (stackDepth != 0 && stackDepth != 1 && stackDepth != 4 && stackDepth != 16)
         return fail(MLBVH_ERR_INVALID_ARG, "stackDepth must be 0, 1, 4 or 16");
     if (nRays >= (1u << 30) && dCounts) return fail(MLBVH_ERR_INVALID_ARG, "nRays must be below 2^30 with counts");
-    const unsigned blocks = (nRays + kTraceThreads - 1) / kTraceThreads;
     const float4* rays = reinterpret_cast<const float4*>(dRays);
     float4* hits = reinterpret_cast<float4*>(dHits);
     if (rayQuery == MLBVH_RAY_QUERY_ANY)
-        launch_trace_quantised_depth<true>(stackDepth, blocks, stream, dQNodes, dQParents, dQTris, dQHeader, rays, hits,
+        launch_trace_quantised_depth<true>(stackDepth, stream, dQNodes, dQParents, dQTris, dQHeader, rays, hits,
                                            nRays, dCounts);
     else
-        launch_trace_quantised_depth<false>(stackDepth, blocks, stream, dQNodes, dQParents, dQTris, dQHeader, rays,
+        launch_trace_quantised_depth<false>(stackDepth, stream, dQNodes, dQParents, dQTris, dQHeader, rays,
                                             hits, nRays, dCounts);
     MLBVH_CHECK_LAUNCH("k_trace_quantised");
     return MLBVH_OK;

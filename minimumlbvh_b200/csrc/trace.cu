@@ -1,39 +1,69 @@
-// Ray queries over the reference node layout: one thread per ray.
+// Ray queries over the reference node layout.
 //
 // Replaces the per-ray device calls of intersect_stackfree (minimum_lbvh.h:
 // 981-1061), intersect_escape_link (:1063-1137) and intersect_stackfull
 // (:912-973) with a single launch. MLBVH_TRAVERSAL_STACKFREE and
 // MLBVH_TRAVERSAL_REPLAY both run the replay walk, which returns
 // intersect_stackfree's Hit records bit for bit and loads every node once
-// instead of up to three times (1M camera rays of a 4M-triangle soup 0.690 ->
-// 0.505 ms, 4,099 rays over 20,011 triangles 56.3 -> 41.6 us). Rays and hits
-// move as 2 x 16-byte vectors, nodes as 2 x 32-byte read-only loads.
+// instead of up to three times (one ray per thread, 1M camera rays of a
+// 4M-triangle soup: 0.690 -> 0.505 ms), scheduled by ray_pool.cuh. Rays and
+// hits move as 2 x 16-byte vectors, nodes as 2 x 32-byte read-only loads.
 #include "capi_internal.h"
 #include "../../include/mlbvh_device.cuh"
+#include "ray_pool.cuh"
 
 namespace mlbvh {
 
 namespace {
 
-// Threads per CTA: a CTA holds its slot until its longest ray is done, so
-// smaller CTAs free slots sooner (measured on 1M camera rays of the 4M soup,
-// replay / stack-free walk: 128 threads 0.552 / 0.689 ms, 64 0.505 / 0.690,
-// 32 0.522 / 0.719; on 1M random rays 1.38 / 1.61, 1.275 / 1.58, 1.29 / 1.65).
-// Build-time override for sweeps: -DMLBVH_TRACE_THREADS.
-#ifndef MLBVH_TRACE_THREADS
-#define MLBVH_TRACE_THREADS 64
-#endif
-constexpr int kTraceThreads = MLBVH_TRACE_THREADS;
+constexpr int kNodeSteps = 4;  // node visits per leaf test (2-4 within 4 %)
+constexpr int kPoolWarps = 32;  // resident warps per SM of the pooled trace kernel (64 registers)
+
+constexpr int kTraceThreads = 64;  // of the one-ray-per-thread walks
 
 constexpr int kReplayDepth = 16;  // stack entries per ray of the replay walk
 
+// intersect_stackfree's Hit records through the replay walk.
+template <bool kAny>
+__global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
+    k_trace_replay(const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
+                   const float* __restrict__ tris, const float4* __restrict__ rays, float4* __restrict__ hits,
+                   RayPool pool)
+{
+    __shared__ typename ReplayStack<kAny>::Entry s_stack[kReplayDepth][kPoolThreads];
+    const uint32_t root = __ldg(rootPtr);
+    f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
+    float tmin = 0.0f;
+    HitRecord hit;
+    uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0;
+    int depth = 0;
+    trace_pool<kNodeSteps>(
+        rays, hits, pool, hit, curr,
+        [&](uint32_t, float4 a, float4 b) {
+            ro = mk(a.x, a.y, a.z);
+            rd = mk(b.x, b.y, b.z);
+            inv = inv_rd(rd);
+            tmin = a.w;
+            hit = HitRecord{b.w, 0.0f, 0.0f, mk(0.0f, 0.0f, 0.0f), 0xFFFFFFFFu};
+            curr = root;
+            prev = kInvalid;
+            depth = 0;
+        },
+        [&] { return depth < 0; },
+        [&] {
+            return stackfree_replay_step<kAny, false, kReplayDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
+                                                                    kPoolThreads, hit, nodes, tris, ro, rd, inv, tmin,
+                                                                    nv, nt);
+        },
+        [](uint32_t) {});
+}
+
+// The reference's other walks, one ray per thread.
 template <int kMode, bool kAny>
 __global__ void __launch_bounds__(kTraceThreads)
     k_trace(const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
             const float* __restrict__ tris, const float4* __restrict__ rays, float4* __restrict__ hits, uint32_t n)
 {
-    __shared__ typename ReplayStack<kAny>::Entry s_stack[kMode == MLBVH_TRAVERSAL_REPLAY ? kReplayDepth : 1]
-                                                        [kTraceThreads];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
@@ -49,14 +79,6 @@ __global__ void __launch_bounds__(kTraceThreads)
     const f3 inv = inv_rd(rd);
     if (kMode == MLBVH_TRAVERSAL_ESCAPE_LINK) {
         trace_escape<kAny>(hit, nodes, tris, root, ro, rd, inv, tmin);
-    } else if (kMode == MLBVH_TRAVERSAL_REPLAY) {
-        uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0;
-        int depth = 0;
-        for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps)
-            if (stackfree_replay_step<kAny, false, kReplayDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                                 kTraceThreads, hit, nodes, tris, ro, rd, inv, tmin,
-                                                                 nv, nt))
-                break;
     } else {
         uint32_t stack[64];
         trace_stackfull(hit, nodes, tris, root, ro, rd, inv, tmin, stack, 64);
@@ -90,12 +112,14 @@ mlbvh_status trace(const mlbvh_internal_node* dNodes, const mlbvh_node_index* dR
             k_trace<MLBVH_TRAVERSAL_ESCAPE_LINK, false><<<blocks, kTraceThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, nRays);
         break;
     case MLBVH_TRAVERSAL_STACKFREE:  // the replay walk's Hit records are the stack-free walk's
-    case MLBVH_TRAVERSAL_REPLAY:
+    case MLBVH_TRAVERSAL_REPLAY: {
+        const RayPool pool = ray_pool(nRays, device_sm_count(), kPoolWarps);
         if (any)
-            k_trace<MLBVH_TRAVERSAL_REPLAY, true><<<blocks, kTraceThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, nRays);
+            k_trace_replay<true><<<pool.ctas, kPoolThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, pool);
         else
-            k_trace<MLBVH_TRAVERSAL_REPLAY, false><<<blocks, kTraceThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, nRays);
+            k_trace_replay<false><<<pool.ctas, kPoolThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, pool);
         break;
+    }
     case MLBVH_TRAVERSAL_STACKFULL:
         k_trace<MLBVH_TRAVERSAL_STACKFULL, false><<<blocks, kTraceThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, nRays);
         break;

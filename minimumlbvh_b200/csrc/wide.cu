@@ -7,17 +7,17 @@
 // which name the slots of their own expansions.
 #include "capi_internal.h"
 #include "../../include/mlbvh_device.cuh"
+#include "ray_pool.cuh"
 
 namespace mlbvh {
 namespace {
 
 constexpr int kWideThreads = 256;
-// threads per CTA of the wide trace kernel (build-time override for sweeps: -DMLBVH_WIDE_TRACE_THREADS=...)
-#ifndef MLBVH_WIDE_TRACE_THREADS
-#define MLBVH_WIDE_TRACE_THREADS 128
-#endif
-constexpr int kWideTraceThreads = MLBVH_WIDE_TRACE_THREADS;
-
+constexpr int kReplayDepth = 16;  // stack entries of the binary replay walk
+// resident warps per SM of the trace kernel, closest hit and any hit
+template <bool kAny>
+constexpr int kPoolWarps = kAny ? 32 : 28;  // (24 / 28 / 32, closest: camera rays 401 / 373 / 413 us, quantised 464 / 437 / 512)
+constexpr int kNodeSteps = 3;  // slot visits per leaf test (2 and 4 within 3 %)
 struct WideKid {
     uint32_t name;  // internal index, kLeafBit | leaf position, or kWideEmpty
     f3 lo, hi;
@@ -178,59 +178,75 @@ __global__ void __launch_bounds__(kWideThreads)
     reinterpret_cast<uint4*>(dst)[3] = ch;
 }
 
-// One thread per ray, any-hit (wide_any_step) or closest-hit
+// The rays of a pool (ray_pool.cuh), any-hit (wide_any_step) or closest-hit
 // (wide_closest_step), over FP32 slots or (kQuant) quantised slots. counts
 // (may be null): per ray, node visits, triangle tests and restarts at
-// counts[i], counts[n + i], counts[2n + i]. status (quantised slots): nonzero
-// sends every ray to the stack-free walk over the binary tree; so does a ray
-// that qwide_ray_fits rejects.
+// counts[i], counts[pool.n + i], counts[2n + i]. status (quantised slots): nonzero
+// sends every ray to the binary tree, and qwide_ray_fits the rays it rejects:
+// to the stack-free walk, or for closest hits without counters to the replay
+// walk, which returns the same Hit records.
 template <bool kAny, bool kCount, bool kQuant, class Slot>
-__global__ void __launch_bounds__(kWideTraceThreads)
+__global__ void __launch_bounds__(kPoolThreads, kPoolWarps<kAny> * 32 / kPoolThreads)
     k_trace_wide(const Slot* __restrict__ slots, const uint32_t* __restrict__ status,
                  const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
                  const float* __restrict__ tris, const mlbvh_qtri* __restrict__ leafTris,
-                 const float4* __restrict__ rays, float4* __restrict__ hits, uint32_t n,
-                 uint32_t* __restrict__ counts)
+                 const float4* __restrict__ rays, float4* __restrict__ hits,
+                 uint32_t* __restrict__ counts, RayPool pool)
 {
     using Entry = typename ReplayStack<kAny>::Entry;
-    __shared__ Entry s_stack[kWideDepth][kWideTraceThreads];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
-    const f3 ro = mk(a.x, a.y, a.z), rd = mk(b.x, b.y, b.z);
-    HitRecord hit;
-    hit.t = b.w;
-    hit.u = 0.0f;
-    hit.v = 0.0f;
-    hit.ng = mk(0.0f, 0.0f, 0.0f);
-    hit.tri = 0xFFFFFFFFu;
+    __shared__ Entry s_stack[kWideDepth][kPoolThreads];
     const uint32_t root = __ldg(rootPtr);
-    const f3 inv = inv_rd(rd);
-    uint32_t nv = 0, nt = 0, nr = 0;
-    uint32_t curr = (root & kLeafBit) ? kLeafBit : root, prev = kInvalid;
+    const bool unusable = kQuant && __ldg(status) != 0u;
+    f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
+    float tmin = 0.0f;
+    HitRecord hit;
+    uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0, nr = 0;
     int depth = 0;
-    if (kQuant && (__ldg(status) != 0u || !qwide_ray_fits(ro, inv))) {
-        curr = root;
-        depth = -1;
-    }
-    for (uint32_t steps = 1; steps < kMaxTraversalSteps; ++steps) {
-        bool done;
-        if constexpr (kAny)
-            done = wide_any_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kWideTraceThreads, hit,
-                                                 slots, nodes, tris, leafTris, root, ro, rd, inv, a.w, nv, nt, nr);
-        else
-            done = wide_closest_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kWideTraceThreads,
-                                                     hit, slots, nodes, tris, leafTris, root, ro, rd, inv, a.w, nv,
-                                                     nt, nr);
-        if (done) break;
-    }
-    hits[2 * (size_t)i] = make_float4(hit.t, 0.0f, hit.u, hit.v);
-    hits[2 * (size_t)i + 1] = make_float4(hit.ng.x, hit.ng.y, hit.ng.z, __uint_as_float(hit.tri));
-    if (kCount) {
-        counts[i] = nv;
-        counts[n + i] = nt;
-        counts[2 * (size_t)n + i] = nr;
-    }
+    constexpr bool kReplayBinary = kQuant && !kAny && !kCount;
+    bool binary = false;  // this ray walks the binary tree
+    trace_pool<kNodeSteps>(
+        rays, hits, pool, hit, curr,
+        [&](uint32_t, float4 a, float4 b) {
+            ro = mk(a.x, a.y, a.z);
+            rd = mk(b.x, b.y, b.z);
+            inv = inv_rd(rd);
+            tmin = a.w;
+            hit = HitRecord{b.w, 0.0f, 0.0f, mk(0.0f, 0.0f, 0.0f), 0xFFFFFFFFu};
+            curr = (root & kLeafBit) ? kLeafBit : root;
+            prev = kInvalid;
+            depth = 0;
+            if (kQuant && (unusable || !qwide_ray_fits(ro, inv))) {
+                curr = root;
+                if (kReplayBinary)
+                    binary = true;
+                else
+                    depth = -1;
+            } else if (kReplayBinary) {
+                binary = false;
+            }
+            if (kCount) nv = nt = nr = 0;
+        },
+        [&] { return depth < 0 || (kReplayBinary && binary); },
+        [&] {
+            if (kReplayBinary && binary)
+                return stackfree_replay_step<kAny, kCount, kReplayDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
+                                                                         kPoolThreads, hit, nodes, tris, ro, rd, inv,
+                                                                         tmin, nv, nt);
+            if constexpr (kAny)
+                return wide_any_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kPoolThreads, hit,
+                                                     slots, nodes, tris, leafTris, root, ro, rd, inv, tmin, nv, nt, nr);
+            else
+                return wide_closest_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kPoolThreads,
+                                                         hit, slots, nodes, tris, leafTris, root, ro, rd, inv, tmin,
+                                                         nv, nt, nr);
+        },
+        [&](uint32_t i) {
+            if (kCount) {
+                counts[i] = nv;
+                counts[pool.n + i] = nt;
+                counts[2 * (size_t)pool.n + i] = nr;
+            }
+        });
 }
 
 inline bool aligned128(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 127u) == 0; }
@@ -270,23 +286,23 @@ mlbvh_status launch_trace_wide(const Slot* dSlots, const uint32_t* dStatus, cons
         return fail(MLBVH_ERR_INVALID_ARG,
                     "device pointers misaligned (wide slots 128 B, quantised slots and nodes 32 B, others 16 B)");
     if (nRays >= (1u << 30) && dCounts) return fail(MLBVH_ERR_INVALID_ARG, "nRays must be below 2^30 with counts");
-    const unsigned blocks = (nRays + kWideTraceThreads - 1) / kWideTraceThreads;
     const float4* rays = reinterpret_cast<const float4*>(dRays);
     float4* hits = reinterpret_cast<float4*>(dHits);
     const float* tris = reinterpret_cast<const float*>(dTris);
     const bool any = rayQuery == MLBVH_RAY_QUERY_ANY;
+    const RayPool pool = ray_pool(nRays, device_sm_count(), any ? kPoolWarps<true> : kPoolWarps<false>);
     if (any && dCounts)
-        k_trace_wide<true, true, kQuant><<<blocks, kWideTraceThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nRays, dCounts);
+        k_trace_wide<true, true, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
+            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, dCounts, pool);
     else if (any)
-        k_trace_wide<true, false, kQuant><<<blocks, kWideTraceThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nRays, nullptr);
+        k_trace_wide<true, false, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
+            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nullptr, pool);
     else if (dCounts)
-        k_trace_wide<false, true, kQuant><<<blocks, kWideTraceThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nRays, dCounts);
+        k_trace_wide<false, true, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
+            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, dCounts, pool);
     else
-        k_trace_wide<false, false, kQuant><<<blocks, kWideTraceThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nRays, nullptr);
+        k_trace_wide<false, false, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
+            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nullptr, pool);
     MLBVH_CHECK_LAUNCH("k_trace_wide");
     return MLBVH_OK;
 }
