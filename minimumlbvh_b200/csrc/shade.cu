@@ -116,26 +116,6 @@ __device__ __forceinline__ bool tile_pixel(int w, int h, int& xi, int& yi)
     return xi < w && yi < h;
 }
 
-// The path tracer's own tiles: kPtWarps warps of 8 x 4 pixels (1: 8 x 4,
-// 2: 16 x 4, 4: 16 x 8, the other kernels' tile). A CTA holds its slot until
-// its longest path is done, and Russian roulette makes path lengths differ
-// widely; measured on the bench's PT pass (replay walk): 0.615 / 0.621 / 0.626
-// ms (build-time override for sweeps: -DMLBVH_PT_WARPS).
-#ifndef MLBVH_PT_WARPS
-#define MLBVH_PT_WARPS 1
-#endif
-constexpr int kPtWarps = MLBVH_PT_WARPS;
-static_assert(kPtWarps == 1 || kPtWarps == 2 || kPtWarps == 4, "1, 2 or 4 warps per path-tracing tile");
-constexpr int kPtThreads = 32 * kPtWarps;
-constexpr int kPtTileW = kPtWarps >= 2 ? 16 : 8, kPtTileH = kPtWarps == 4 ? 8 : 4;
-__device__ __forceinline__ bool pt_pixel(int w, int h, int& xi, int& yi)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    xi = blockIdx.x * kPtTileW + (lane & 7) + 8 * (warp & 1);
-    yi = blockIdx.y * kPtTileH + (lane >> 3) + 4 * (warp >> 1);
-    return xi < w && yi < h;
-}
-
 // PCG32 jump-ahead by `delta` steps (Brown, "Random Number Generation with
 // Arbitrary Strides", 1994), so that AO sample i can start at draw 2i.
 __device__ __forceinline__ void pcg_advance(Pcg& r, uint64_t delta)
@@ -717,13 +697,28 @@ __global__ void __launch_bounds__(kTileW* kTileH)
     pixels[xi + yi * w] = rgba;
 }
 
+// The path tracer's sample stream: Sobol points by dimension, or the PCG
+// stream's numbers in pairs.
+template <bool kSobol>
 struct PtRandom {
-    int useSobol;
-    uint32_t iteration, xi, yi, dim;
-    Pcg rng;
-    __device__ __forceinline__ float2 next()
+    uint32_t dim;
+    __device__ __forceinline__ PtRandom() : dim(0) {}
+    __device__ __forceinline__ PtRandom(int, int) : dim(0) {}
+    __device__ __forceinline__ float2 next(int iteration, int xi, int yi)
     {
-        if (useSobol) return sobol2d(iteration, xi, yi, dim++);
+        return sobol2d((uint32_t)iteration, (uint32_t)xi, (uint32_t)yi, dim++);
+    }
+};
+template <>
+struct PtRandom<false> {
+    Pcg rng;
+    __device__ __forceinline__ PtRandom() : rng(0, 0) {}
+    __device__ __forceinline__ PtRandom(int pixel, int iteration)
+        : rng(hash_pcg(hash_pcg((uint32_t)pixel) + (uint32_t)iteration), 0)
+    {
+    }
+    __device__ __forceinline__ float2 next(int, int, int)
+    {
         float2 r;
         r.x = rng.uniformf();
         r.y = rng.uniformf();
@@ -731,72 +726,153 @@ struct PtRandom {
     }
 };
 
+// Swept on a pass over the heightfield at 512x512 / 1024x768 (us; one thread per
+// pixel, nodes and leaves in phases: 646 / -): warps per SM 20 589 / 1,097, 24
+// 552 / 1,034, 28 (72 registers) 539 / 996, 32 542 / 980; CTAs of 64 threads 579
+// / 1,077; 3 node visits 559 / 1,071; 4 waiting lanes 558 / 1,080, 12 557 /
+// 1,042. A 64x64 pass takes 221: its longest path, which is also what the
+// larger passes end with.
+constexpr int kPtThreads = 128;
+constexpr int kPtWarps = 28;   // resident warps per SM the kernel is compiled for
+constexpr int kPtSteps = 4;    // node visits per leaf test
+constexpr int kPtService = 8;  // lanes that wait for their next ray before it is set up
+
+// The launch of a pass: a CTA takes tiles of 8 x 4 pixels, tile t CTA t modulo
+// their number (neighbouring paths cost alike); where it has fewer pixels than
+// lanes its warps share them out.
+struct PtPool {
+    int w, h;
+    uint32_t tilesX, tiles, ctas, lanes;
+};
+
 // pt (main_gpu.cu:179-272): one progressive sample per pixel. Tree: the
-// walk of every closest-hit ray (PlainTree: intersect_stackfree as the
-// reference; the replay trees: the same Hit records from a per-thread stack
-// of pending far children in shared memory), so the accumulators are the same.
-template <class Tree>
-__global__ void __launch_bounds__(kPtThreads)
-    k_pt(float4* __restrict__ accum, mlbvh_ray_generator gen, int w, int h, Tree tree,
-         const float* __restrict__ attribs, int useSobol, int maxSPP, int maxDepth)
+// walk of every closest-hit ray (the replay trees: intersect_stackfree's Hit
+// records from a per-thread stack of pending far children in shared memory).
+// Every lane traces a path of its own; a lane whose ray is done waits until
+// kPtService lanes do (or as many as still walk), and those lanes shade
+// together, go on with their paths' next rays or take the CTA's next pixels: path
+// lengths differ widely (Russian roulette).
+template <class Tree, bool kSobol>
+__global__ void __launch_bounds__(kPtThreads, kPtWarps * 32 / kPtThreads)
+    k_pt(float4* __restrict__ accum, mlbvh_ray_generator gen, PtPool pool, Tree tree,
+         const float* __restrict__ attribs, int maxSPP, int maxDepth)
 {
-    __shared__ uint2 s_pstack[Tree::kPrimaryStack > 0 ? Tree::kPrimaryStack : 1][kPtThreads];
+    __shared__ uint2 s_pstack[Tree::kPrimaryStack][kPtThreads];
+    __shared__ uint32_t s_next;
+    if (threadIdx.x == 0) s_next = 0;
+    __syncthreads();
     uint2* const pstack = &s_pstack[0][threadIdx.x];
     Counts cnt;
-    int xi, yi;
-    if (!pt_pixel(w, h, xi, yi)) return;
     const Camera cam = to_camera(gen);
-    const int pixel = xi + yi * w;
-    float4 acc = accum[pixel];
-    const int iteration = (int)acc.w;
-    PtRandom rr{useSobol, (uint32_t)iteration, (uint32_t)xi, (uint32_t)yi, 0u,
-                Pcg(hash_pcg(hash_pcg((uint32_t)pixel) + (uint32_t)iteration), 0)};
     const typename Tree::Ctx ctx = tree.context();
-    float2 rnd = rr.next();
-    f3 ro, rd;
-    shoot(cam, ((float)xi + rnd.x) / (float)w, ((float)yi + rnd.y) / (float)h, ro, rd);
-    f3 color = mk(0.0f, 0.0f, 0.0f);
-    f3 throughput = mk(1.0f, 1.0f, 1.0f);
+    const uint32_t lane = threadIdx.x & 31;
+    const bool used = lane < pool.lanes;
+    const uint32_t mine = 32 * ((pool.tiles - blockIdx.x + pool.ctas - 1) / pool.ctas);
+    bool more = true;                   // warp-uniform: the CTA has pixels left
+    bool path = false, walking = false;  // the lane has a path; its ray is in flight
+    int xi = 0, yi = 0, iteration = 0, bounce = 0;
+    PtRandom<kSobol> rr;
+    f3 ro = mk(0, 0, 0), rd = ro, inv = ro, color = ro, throughput = ro;
     HitRecord hit;
     hit.t = kFltMax;
-    hit.tri = 0xFFFFFFFFu;
-    tree.template trace<false, false>(ctx, hit, ro, rd, cnt, pstack, kPtThreads);
-    if (hit.t != kFltMax)
-        for (int depth = 0; depth < maxDepth; depth++) {
-            const float2 r2 = rr.next();
-            const f3 hit_p = ro + rd * hit.t;
-            f3 hit_n = normalize(hit.ng);
-            if (0.0f < dot(hit_n, rd)) hit_n = -hit_n;
-            const float* at = attribs + 15 * (size_t)hit.tri;
-            const f3 refl = mk(__ldg(at + 9), __ldg(at + 10), __ldg(at + 11));
-            const f3 emis = mk(__ldg(at + 12), __ldg(at + 13), __ldg(at + 14));
-            color = color + throughput * emis;
-            f3 xaxis, zaxis;
-            onb(hit_n, xaxis, zaxis);
-            const f3 dl = sample_hemisphere(r2.x, r2.y);
-            const f3 next_ro = hit_p + hit_n * 0.0001f;
-            const f3 next_rd = xaxis * dl.x + zaxis * dl.z + hit_n * dl.y;
-            throughput = throughput * refl;
-            const float rrThreshold = 0.25f;
-            const float maxComp = smax(smax(throughput.x, throughput.y), throughput.z);
-            const float p = smin(maxComp / rrThreshold, 1.0f);
-            if (p < rr.next().x) break;
-            throughput = throughput / p;
-            hit.t = kFltMax;
-            hit.u = hit.v = 0.0f;
-            hit.ng = mk(0.0f, 0.0f, 0.0f);
-            hit.tri = 0xFFFFFFFFu;
-            tree.template trace<false, false>(ctx, hit, next_ro, next_rd, cnt, pstack, kPtThreads);
-            if (hit.t == kFltMax) break;
-            ro = next_ro;
-            rd = next_rd;
+    hit.tri = 0;
+    hit.ng = ro;
+    uint32_t curr = 0, prev = 0, steps = 0;
+    int depth = 0;
+    for (;;) {
+        const int walkers = __popc(__ballot_sync(0xffffffffu, walking));
+        const int waiting = __popc(__ballot_sync(0xffffffffu, used && !walking && (path || more)));
+        if (walkers == 0 && waiting == 0) return;
+        if (waiting >= min(kPtService, max(walkers, 1))) {
+            bool start = false;
+            if (path && !walking) {
+                bool ended = hit.t == kFltMax || bounce == maxDepth;
+                if (!ended) {
+                    const float2 r2 = rr.next(iteration, xi, yi);
+                    const f3 hit_p = ro + rd * hit.t;
+                    f3 hit_n = normalize(hit.ng);
+                    if (0.0f < dot(hit_n, rd)) hit_n = -hit_n;
+                    const float* at = attribs + 15 * (size_t)hit.tri;
+                    const f3 refl = mk(__ldg(at + 9), __ldg(at + 10), __ldg(at + 11));
+                    const f3 emis = mk(__ldg(at + 12), __ldg(at + 13), __ldg(at + 14));
+                    color = color + throughput * emis;
+                    f3 xaxis, zaxis;
+                    onb(hit_n, xaxis, zaxis);
+                    const f3 dl = sample_hemisphere(r2.x, r2.y);
+                    ro = hit_p + hit_n * 0.0001f;
+                    rd = xaxis * dl.x + zaxis * dl.z + hit_n * dl.y;
+                    throughput = throughput * refl;
+                    const float rrThreshold = 0.25f;
+                    const float maxComp = smax(smax(throughput.x, throughput.y), throughput.z);
+                    const float p = smin(maxComp / rrThreshold, 1.0f);
+                    if (p < rr.next(iteration, xi, yi).x) {
+                        ended = true;
+                    } else {
+                        throughput = throughput / p;
+                        ++bounce;
+                        start = true;
+                    }
+                }
+                if (ended) {
+                    path = false;
+                    if (iteration < maxSPP) {
+                        float4 acc = accum[xi + yi * pool.w];
+                        acc.x += color.x;
+                        acc.y += color.y;
+                        acc.z += color.z;
+                        acc.w += 1.0f;
+                        accum[xi + yi * pool.w] = acc;
+                    }
+                }
+            }
+            // ---- lanes without a path take the CTA's next pixels
+            const uint32_t idle = __ballot_sync(0xffffffffu, used && !path);
+            if (more && idle) {
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(&s_next, (uint32_t)__popc(idle));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                more = base + __popc(idle) < mine;
+                const uint32_t j = base + __popc(idle & ((1u << lane) - 1u));
+                if (used && !path && j < mine) {
+                    const uint32_t tile = (j >> 5) * pool.ctas + blockIdx.x;
+                    xi = (int)(tile % pool.tilesX * 8 + (j & 7u));
+                    yi = (int)(tile / pool.tilesX * 4 + (j >> 3 & 3u));
+                    if (xi < pool.w && yi < pool.h) {
+                        iteration = (int)accum[xi + yi * pool.w].w;
+                        rr = PtRandom<kSobol>(xi + yi * pool.w, iteration);
+                        const float2 rnd = rr.next(iteration, xi, yi);
+                        shoot(cam, ((float)xi + rnd.x) / (float)pool.w, ((float)yi + rnd.y) / (float)pool.h, ro, rd);
+                        color = mk(0.0f, 0.0f, 0.0f);
+                        throughput = mk(1.0f, 1.0f, 1.0f);
+                        bounce = 0;
+                        path = start = true;
+                    }
+                }
+            }
+            if (start) {
+                inv = inv_rd(rd);
+                hit.t = kFltMax;
+                hit.u = hit.v = 0.0f;
+                hit.ng = mk(0.0f, 0.0f, 0.0f);
+                hit.tri = 0xFFFFFFFFu;
+                curr = ctx.root;
+                prev = kInvalid;
+                depth = 0;
+                steps = 0;
+                walking = true;
+            }
         }
-    if (iteration < maxSPP) {
-        acc.x += color.x;
-        acc.y += color.y;
-        acc.z += color.z;
-        acc.w += 1.0f;
-        accum[pixel] = acc;
+        // ---- node visits, then the leaf tests
+        bool done = false;
+        auto step = [&] {
+            return tree.template walk<false, false>(curr, prev, depth, pstack, kPtThreads, hit, ro, rd, inv, cnt);
+        };
+#pragma unroll
+        for (int k = 0; k < kPtSteps; ++k)
+            if (walking && !done && !(curr & kLeafBit) && depth >= 0) done = step();
+        if (walking && !done && ((curr & kLeafBit) || depth < 0)) done = step();
+        steps += kPtSteps + 1;
+        if (done || steps >= kMaxTraversalSteps) walking = false;
     }
 }
 
@@ -1005,14 +1081,22 @@ mlbvh_status render_pt(float* dAccum, int w, int h, const mlbvh_ray_generator& c
     float4* acc = reinterpret_cast<float4*>(dAccum);
     const float* tris = reinterpret_cast<const float*>(dTris);
     const float* at = reinterpret_cast<const float*>(dAttribs);
-    const dim3 grid((unsigned)((w + kPtTileW - 1) / kPtTileW), (unsigned)((h + kPtTileH - 1) / kPtTileH));
-    // both walks take the replay kernel: the same accumulators (heightfield, 512x512: 0.90 -> 0.71 ms)
+    PtPool pool{w, h, (uint32_t)(w + 7) / 8, 0, 0, 32};
+    pool.tiles = pool.tilesX * ((uint32_t)(h + 3) / 4);
+    pool.ctas = std::min(pool.tiles, (uint32_t)device_sm_count() * (uint32_t)(kPtWarps * 32 / kPtThreads));
+    const uint32_t perCta = 32 * ((pool.tiles + pool.ctas - 1) / pool.ctas);
+    pool.lanes = std::min(32u, (perCta + kPtThreads / 32 - 1) / (kPtThreads / 32));
+    auto launch = [&](auto tree) {  // both walks take the replay kernel: the same accumulators
+        if (useSobol)
+            k_pt<decltype(tree), true><<<pool.ctas, kPtThreads, 0, stream>>>(acc, cam, pool, tree, at, maxSPP, maxDepth);
+        else
+            k_pt<decltype(tree), false><<<pool.ctas, kPtThreads, 0, stream>>>(acc, cam, pool, tree, at, maxSPP,
+                                                                              maxDepth);
+    };
     if (traversal == MLBVH_TRAVERSAL_REPLAY && dLeafTris)
-        k_pt<<<grid, kPtThreads, 0, stream>>>(acc, cam, w, h, PlainReplayLeafTree{dNodes, tris, dRoot, dLeafTris},
-                                                   at, useSobol, maxSPP, maxDepth);
+        launch(PlainReplayLeafTree{dNodes, tris, dRoot, dLeafTris});
     else
-        k_pt<<<grid, kPtThreads, 0, stream>>>(acc, cam, w, h, PlainReplayTree{dNodes, tris, dRoot, nullptr}, at,
-                                                   useSobol, maxSPP, maxDepth);
+        launch(PlainReplayTree{dNodes, tris, dRoot, nullptr});
     MLBVH_CHECK_LAUNCH("k_pt");
     return MLBVH_OK;
 }
