@@ -66,8 +66,12 @@ namespace mlbvh {
 namespace {
 
 constexpr int kPlocThreads = sort::kThreads;  // 256 (block_scan's width)
-constexpr int kPer = 4;                       // clusters per thread in a tile
+constexpr int kPer = 4;                       // clusters per thread in a large tile
 constexpr uint32_t kTile = kPlocThreads * kPer;
+// At most this many clusters (fewer large tiles than multiprocessors) are cut
+// into small tiles of one cluster per thread: a quarter of the search per
+// thread, on four times the multiprocessors.
+constexpr uint32_t kSmallMax = 148 * kTile;
 constexpr uint32_t kTailClusters = kTile;
 constexpr int kMaxRadius = 32;
 constexpr uint32_t kSpan = kTile + 2 * kMaxRadius;  // staged clusters per tile (kTile - 2r + 4r)
@@ -88,12 +92,13 @@ constexpr unsigned long long kValueMask = (1ull << 62) - 1;
 constexpr int kMergeShift = 31;  // packed counts: survivors bits 0-30, merges bits 31-61
 constexpr unsigned long long kCountMask = (1ull << 31) - 1;
 
-// clusters / merged after grid-phase iteration k sit in slot (k + 1) & 1: the
-// last tile of iteration k writes them while a CTA without tiles may still be
-// reading slot k & 1, and cannot read slot (k + 1) & 1 before the barrier.
+// One word counts an iteration's arrivals (bits 48-63), those with an error
+// (bits 31-47) and takes the survivors from the CTA of the last tile (bits
+// 0-30); the last to arrive publishes the next iteration's number (bits 32-63)
+// with the survivors (~0: stop) in another, which the others poll.
 struct PlocControl {
-    uint32_t barrierCount, barrierGen;
-    uint32_t clusters[2], merged[2];
+    unsigned long long arrivals, release;
+    uint32_t done;       // 1: the tree is made, place it; 2: stop
     uint32_t placeNext;  // next position of the placement order to hand out
 };
 
@@ -121,7 +126,8 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 PlocLayout ploc_layout(uint32_t n)
 {
     PlocLayout L;
-    L.maxTiles = (n + (kTile - 2 * kMaxRadius) - 1) / (kTile - 2 * kMaxRadius);
+    constexpr uint32_t kBig = kTile - 2 * kMaxRadius, kSmall = kPlocThreads - 2 * kMaxRadius;
+    L.maxTiles = std::max((n + kBig - 1) / kBig, (std::min(n, kSmallMax) + kSmall - 1) / kSmall);
     size_t o = align256(build_scratch_bytes(n));
     L.control = o;
     o += 256;
@@ -148,6 +154,16 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p)
 __device__ __forceinline__ void st_release(uint32_t* p, uint32_t v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release64(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long* p)
 {
@@ -216,6 +232,7 @@ __device__ __noinline__ uint32_t resolve_tie(uint32_t p, uint32_t bestA, uint32_
 // positions cut off that way are not written). Keys are at most +inf's bits,
 // so the first candidate always beats the initial 0xFFFFFFFF and ascending j
 // keeps the smaller position on ties.
+template <int kPer>
 __device__ __forceinline__ void nearest_group(uint32_t p0, uint32_t first, uint32_t end, uint32_t base,
                                               uint32_t staged, int r, const float4* sLo, const float4* sHi,
                                               uint32_t* sNN)
@@ -255,7 +272,7 @@ __device__ __forceinline__ void nearest_group(uint32_t p0, uint32_t first, uint3
 // nearest_group with the radius fixed at compile time, for groups whose whole
 // window [p0 - R, p0 + kPer - 1 + R] is staged: the loops unroll and every
 // window test resolves at compile time.
-template <int R>
+template <int R, int kPer>
 __device__ __forceinline__ void nearest_fixed(uint32_t p0, uint32_t first, uint32_t end, uint32_t base,
                                               const float4* sLo, const float4* sHi, uint32_t* sNN)
 {
@@ -290,19 +307,20 @@ __device__ __forceinline__ void nearest_fixed(uint32_t p0, uint32_t first, uint3
     }
 }
 
-template <int R>
+template <int R, int kPer>
 __device__ __forceinline__ void nearest(uint32_t p0, uint32_t first, uint32_t end, uint32_t base, uint32_t staged,
                                         int r, const float4* sLo, const float4* sHi, uint32_t* sNN)
 {
     if (R > 0 && p0 >= base + R && p0 + kPer - 1 + R < staged)
-        nearest_fixed<R>(p0, first, end, base, sLo, sHi, sNN);
+        nearest_fixed<R, kPer>(p0, first, end, base, sLo, sHi, sNN);
     else
-        nearest_group(p0, first, end, base, staged, r, sLo, sHi, sNN);
+        nearest_group<kPer>(p0, first, end, base, staged, r, sLo, sHi, sNN);
 }
 
 // A pairing iteration: position 2k's neighbour is 2k + 1 and the other way
 // round; an odd last cluster points back and stays (tiles start at even
 // positions, so no pair straddles two tiles).
+template <int kPer>
 __device__ __forceinline__ void pair_partners(uint32_t p0, uint32_t first, uint32_t end, uint32_t base, uint32_t C,
                                               uint32_t* sNN)
 {
@@ -319,6 +337,7 @@ __device__ __forceinline__ void pair_partners(uint32_t p0, uint32_t first, uint3
 // key of the neighbour found, the one with the smallest pair_hash (the window
 // as nearest_group clamps it). Run after the search, so the unrolled search
 // keeps its registers; it reads boxes and writes only its own entries.
+template <int kPer>
 __device__ __forceinline__ void resolve_ties(uint32_t p0, uint32_t first, uint32_t end, uint32_t base,
                                              uint32_t staged, int r, const float4* sLo, const float4* sHi,
                                              uint32_t* sNN)
@@ -338,6 +357,7 @@ __device__ __forceinline__ void resolve_ties(uint32_t p0, uint32_t first, uint32
 struct Decision {
     uint32_t keepMask, mergeMask;
 };
+template <int kPer>
 __device__ __forceinline__ Decision decide(uint32_t p0, uint32_t end, uint32_t base, const uint32_t* sNN)
 {
     Decision dc{0u, 0u};
@@ -424,34 +444,42 @@ __device__ unsigned long long lookback(unsigned long long* flags, uint32_t t, un
     return excl;
 }
 
-// Grid-wide barrier over the cooperative launch. Returns false (in every
-// thread of the CTA) when its wait gave up or the error word is set.
-__device__ bool grid_barrier(PlocControl* ctl, uint32_t* error, uint32_t spinLimit, int* sFlag)
+// The end of iteration `iter` for its `ctas` participating CTAs: survivors is
+// the next cluster count in the CTA of the last tile and 0 elsewhere. Returns
+// the next count to every thread, kUnset when a wait gave up here or elsewhere.
+// A CTA that the next iteration leaves out may find a later iteration's count,
+// which leaves it out too.
+__device__ uint32_t end_iteration(PlocControl* ctl, uint32_t ctas, uint32_t iter, uint32_t survivors, bool failed,
+                                  uint32_t* error, uint32_t spinLimit, uint32_t* sNext)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
-        const uint32_t gen = ld_acquire(&ctl->barrierGen);
         __threadfence();
-        bool ok = true;
-        if (atomicAdd(&ctl->barrierCount, 1u) == gridDim.x - 1) {
-            atomicExch(&ctl->barrierCount, 0u);
+        const unsigned long long mine = 1ull << 48 | (failed ? 1ull << 31 : 0ull) | survivors;
+        const unsigned long long all = atomicAdd(&ctl->arrivals, mine) + mine;
+        uint32_t next;
+        if ((uint32_t)(all >> 48) == ctas) {
             __threadfence();
-            st_release(&ctl->barrierGen, gen + 1);
+            next = (all >> 31 & 0x1FFFFu) ? kUnset : (uint32_t)(all & kCountMask);
+            st_relaxed64(&ctl->arrivals, 0ull);
+            st_release64(&ctl->release, (unsigned long long)(iter + 1) << 32 | next);
         } else {
+            unsigned long long word;
             uint32_t spins = 0;
-            while (ld_acquire(&ctl->barrierGen) == gen) {
+            while ((uint32_t)((word = ld_acquire64(&ctl->release)) >> 32) < iter + 1) {
                 if (++spins > spinLimit) {
                     atomicOr(error, 1u);
-                    ok = false;
+                    word = kUnset;
                     break;
                 }
-                __nanosleep(64);
+                __nanosleep(20);
             }
+            next = (uint32_t)word;
         }
-        *sFlag = ok && ld_acquire(error) == 0;
+        *sNext = next;
     }
     __syncthreads();
-    return *sFlag != 0;
+    return *sNext;
 }
 
 // What a node's placement reads that does not depend on its parent: its
@@ -560,10 +588,8 @@ __global__ void __launch_bounds__(kInitThreads)
     for (uint32_t i = g; i < nFlags; i += stride) flags[i] = 0ull;
     for (uint32_t i = g; i + 1 < n; i += stride) info[i] = ~0ull;
     if (g == 0) {
-        ctl->barrierCount = 0;
-        ctl->barrierGen = 0;
-        ctl->clusters[0] = ctl->clusters[1] = n;
-        ctl->merged[0] = ctl->merged[1] = 0;
+        ctl->arrivals = ctl->release = 0ull;
+        ctl->done = 0;
         ctl->placeNext = 0;
     }
     for (uint32_t i = g; i < n; i += stride) {
@@ -576,103 +602,152 @@ __global__ void __launch_bounds__(kInitThreads)
     }
 }
 
+// Shared memory of a CTA.
+struct PlocShared {
+    float4 *lo, *hi;  // staged clusters
+    uint32_t* nn;     // their neighbours
+    uint32_t* warp;   // kWarps words
+    LookbackShared* look;
+};
+
+// Tile t of an iteration over C clusters (kPer per thread): clusters from src,
+// survivors to dst, new nodes after the `merged` made so far. The last tile
+// returns the survivors, the others 0; ok = false when a wait gave up.
+template <int R, int kPer>
+__device__ __forceinline__ uint32_t ploc_tile(const PlocArgs& a, const PlocShared& sh, uint32_t t, uint32_t tiles,
+                                              uint32_t C, uint32_t merged, int r, bool pairs, bool hashTies,
+                                              const float4* __restrict__ src, float4* __restrict__ dst,
+                                              unsigned long long* flags, bool& ok)
+{
+    const int tid = threadIdx.x;
+    const uint32_t tileClusters = kPlocThreads * kPer - 2u * r;  // the search range of a tile is kPlocThreads * kPer
+    const uint32_t s = t * tileClusters, e = min(s + tileClusters, C);
+    const uint32_t base = s > 2u * r ? s - 2u * r : 0u;
+    const uint32_t stagedEnd = min(C, e + 2u * r);
+    __syncthreads();  // the previous tile's shared-memory reads are done
+    for (uint32_t k = tid; k < stagedEnd - base; k += kPlocThreads) {
+        sh.lo[pad(k)] = __ldcg(src + 2ull * (base + k));
+        sh.hi[pad(k)] = __ldcg(src + 2ull * (base + k) + 1);
+    }
+    __syncthreads();
+    const uint32_t nnFirst = s > (uint32_t)r ? s - r : 0u, nnEnd = min(C, e + r);
+    const uint32_t g0 = nnFirst + kPer * tid;  // nnEnd - nnFirst <= kPlocThreads * kPer: one group per thread
+    if (g0 < nnEnd) {
+        if (pairs)
+            pair_partners<kPer>(g0, nnFirst, nnEnd, base, C, sh.nn);
+        else
+            nearest<R, kPer>(g0, nnFirst, nnEnd, base, stagedEnd, r, sh.lo, sh.hi, sh.nn);
+    }
+    __syncthreads();
+    if (hashTies && !pairs) {  // uniform over the grid
+        if (g0 < nnEnd) resolve_ties<kPer>(g0, nnFirst, nnEnd, base, stagedEnd, r, sh.lo, sh.hi, sh.nn);
+        __syncthreads();
+    }
+    const uint32_t p0 = s + kPer * tid;
+    const Decision dc = decide<kPer>(p0, e, base, sh.nn);
+    uint32_t total;
+    const uint32_t before = sort::block_scan(__popc(dc.keepMask) | __popc(dc.mergeMask) << 16, sh.warp, &total);
+    const unsigned long long agg =
+        (unsigned long long)(total & 0xFFFFu) | (unsigned long long)(total >> 16) << kMergeShift;
+    bool mine = true;
+    const unsigned long long pre = lookback(flags, t, agg, a.error, a.spinLimit, mine, *sh.look);
+    if (!mine) {  // uniform: every thread took the same waits
+        ok = false;
+        return 0;
+    }
+    uint32_t outPos = (uint32_t)(pre & kCountMask) + (before & 0xFFFFu);
+    uint32_t node = merged + (uint32_t)((pre >> kMergeShift) & kCountMask) + (before >> 16);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        if (!((dc.keepMask >> q) & 1u)) continue;
+        const uint32_t p = p0 + q;
+        float4 lo = sh.lo[pad(p - base)], hi = sh.hi[pad(p - base)];
+        if ((dc.mergeMask >> q) & 1u) {
+            const uint32_t j = sh.nn[pad(p - base)];
+            if (node < a.n - 1)
+                merge_pair(a.tmp, node, lo, hi, sh.lo[pad(j - base)], sh.hi[pad(j - base)], lo, hi);
+            ++node;
+        }
+        if (outPos < C) {
+            dst[2ull * outPos] = lo;
+            dst[2ull * outPos + 1] = hi;
+        }
+        ++outPos;
+    }
+    return t == tiles - 1 ? (uint32_t)(pre & kCountMask) + (total & 0xFFFFu) : 0u;
+}
+
+// One iteration over the C clusters in shared memory (at most kPer per
+// thread); returns the survivors, which replace them.
+template <int R, int kPer>
+__device__ __forceinline__ uint32_t ploc_tail(const PlocArgs& a, const PlocShared& sh, uint32_t C, uint32_t merged,
+                                              int r, bool pairs, bool hashTies)
+{
+    const uint32_t g0 = kPer * threadIdx.x;
+    if (g0 < C) {
+        if (pairs)
+            pair_partners<kPer>(g0, 0, C, 0, C, sh.nn);
+        else
+            nearest<R, kPer>(g0, 0, C, 0, C, r, sh.lo, sh.hi, sh.nn);
+    }
+    __syncthreads();
+    if (hashTies && !pairs) {
+        if (g0 < C) resolve_ties<kPer>(g0, 0, C, 0, C, r, sh.lo, sh.hi, sh.nn);
+        __syncthreads();
+    }
+    const Decision dc = decide<kPer>(g0, C, 0, sh.nn);
+    uint32_t total;
+    const uint32_t before = sort::block_scan(__popc(dc.keepMask) | __popc(dc.mergeMask) << 16, sh.warp, &total);
+    float4 keepLo[kPer], keepHi[kPer];
+    uint32_t node = merged + (before >> 16);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        keepLo[q] = keepHi[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!((dc.keepMask >> q) & 1u)) continue;
+        const uint32_t p = g0 + q;
+        keepLo[q] = sh.lo[pad(p)];
+        keepHi[q] = sh.hi[pad(p)];
+        if ((dc.mergeMask >> q) & 1u) {
+            const uint32_t j = sh.nn[pad(p)];
+            if (node < a.n - 1)
+                merge_pair(a.tmp, node, keepLo[q], keepHi[q], sh.lo[pad(j)], sh.hi[pad(j)], keepLo[q], keepHi[q]);
+            ++node;
+        }
+    }
+    __syncthreads();  // every read of this iteration's clusters is done
+    uint32_t outPos = before & 0xFFFFu;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        if (!((dc.keepMask >> q) & 1u)) continue;
+        sh.lo[pad(outPos)] = keepLo[q];
+        sh.hi[pad(outPos)] = keepHi[q];
+        ++outPos;
+    }
+    __syncthreads();
+    return total & 0xFFFFu;
+}
+
 // R: the radius when it is one of the compiled-in values (its groups take the
 // unrolled search), 0 for any radius (the generic search everywhere).
 template <int R>
 __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc(PlocArgs a)
 {
     extern __shared__ float4 smem[];
-    float4* sLo = smem;
-    float4* sHi = smem + kSpanP;
-    uint32_t* sNN = reinterpret_cast<uint32_t*>(smem + 2 * kSpanP);
     __shared__ uint32_t sWarp[sort::kWarps];
     __shared__ LookbackShared sLook;
-    __shared__ int sFlag;
+    __shared__ uint32_t sNext;
+    const PlocShared sh{smem, smem + kSpanP, reinterpret_cast<uint32_t*>(smem + 2 * kSpanP), sWarp, &sLook};
     const int tid = threadIdx.x;
     const int r = R > 0 ? R : (int)a.radius;
-    const uint32_t tileClusters = kTile - 2u * r;  // the search range of a tile is kTile positions
+    const uint32_t bigTile = kTile - 2u * r, smallTile = kPlocThreads - 2u * r;
 
-    uint32_t C = a.n, merged = 0, iter = 0;
+    uint32_t C = a.n, iter = 0;  // C clusters: n - C merges made
     int cur = 0;
-    bool hashTies = false, pairNext = false;  // the same in every CTA: they follow the cluster counts
-    // ------------------------------------------------------------ grid phase
-    while (C > kTailClusters) {
-        const bool pairs = pairNext;
-        const uint32_t tiles = (C + tileClusters - 1) / tileClusters;
-        unsigned long long* flags = a.flags + (size_t)(iter & 1) * a.maxTiles;
-        unsigned long long* nextFlags = a.flags + (size_t)((iter + 1) & 1) * a.maxTiles;
-        const float4* src = cur ? a.clusters[1] : a.clusters[0];
-        float4* dst = cur ? a.clusters[0] : a.clusters[1];
-        for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-            const uint32_t s = t * tileClusters, e = min(s + tileClusters, C);
-            const uint32_t base = s > 2u * r ? s - 2u * r : 0u;
-            const uint32_t stagedEnd = min(C, e + 2u * r);
-            __syncthreads();  // the previous tile's shared-memory reads are done
-            for (uint32_t k = tid; k < stagedEnd - base; k += kPlocThreads) {
-                sLo[pad(k)] = __ldcg(src + 2ull * (base + k));
-                sHi[pad(k)] = __ldcg(src + 2ull * (base + k) + 1);
-            }
-            __syncthreads();
-            const uint32_t nnFirst = s > (uint32_t)r ? s - r : 0u, nnEnd = min(C, e + r);
-            {
-                const uint32_t g0 = nnFirst + kPer * tid;  // nnEnd - nnFirst <= kTile: one group per thread
-                if (g0 < nnEnd) {
-                    if (pairs)
-                        pair_partners(g0, nnFirst, nnEnd, base, C, sNN);
-                    else
-                        nearest<R>(g0, nnFirst, nnEnd, base, stagedEnd, r, sLo, sHi, sNN);
-                }
-            }
-            __syncthreads();
-            if (hashTies && !pairs) {  // uniform over the grid
-                const uint32_t g0 = nnFirst + kPer * tid;
-                if (g0 < nnEnd) resolve_ties(g0, nnFirst, nnEnd, base, stagedEnd, r, sLo, sHi, sNN);
-                __syncthreads();
-            }
-            const uint32_t p0 = s + kPer * tid;
-            const Decision dc = decide(p0, e, base, sNN);
-            uint32_t total;
-            const uint32_t before = sort::block_scan(__popc(dc.keepMask) | __popc(dc.mergeMask) << 16, sWarp, &total);
-            const unsigned long long agg =
-                (unsigned long long)(total & 0xFFFFu) | (unsigned long long)(total >> 16) << kMergeShift;
-            bool ok = true;
-            const unsigned long long pre = lookback(flags, t, agg, a.error, a.spinLimit, ok, sLook);
-            if (tid == 0) {
-                nextFlags[t] = 0ull;
-                if (t == tiles - 1) {
-                    const uint32_t survivors = (uint32_t)(pre & kCountMask) + (total & 0xFFFFu);
-                    const uint32_t mergedAfter = merged + (uint32_t)((pre >> kMergeShift) & kCountMask) + (total >> 16);
-                    a.ctl->clusters[(iter + 1) & 1] = survivors;
-                    a.ctl->merged[(iter + 1) & 1] = mergedAfter;
-                }
-            }
-            if (!ok) continue;  // uniform: every thread took the same waits
-            uint32_t outPos = (uint32_t)(pre & kCountMask) + (before & 0xFFFFu);
-            uint32_t node = merged + (uint32_t)((pre >> kMergeShift) & kCountMask) + (before >> 16);
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                if (!((dc.keepMask >> q) & 1u)) continue;
-                const uint32_t p = p0 + q;
-                float4 lo = sLo[pad(p - base)], hi = sHi[pad(p - base)];
-                if ((dc.mergeMask >> q) & 1u) {
-                    const uint32_t j = sNN[pad(p - base)];
-                    if (node < a.n - 1)
-                        merge_pair(a.tmp, node, lo, hi, sLo[pad(j - base)], sHi[pad(j - base)], lo, hi);
-                    ++node;
-                }
-                if (outPos < C) {
-                    dst[2ull * outPos] = lo;
-                    dst[2ull * outPos + 1] = hi;
-                }
-                ++outPos;
-            }
-        }
-        if (!grid_barrier(a.ctl, a.error, a.spinLimit, &sFlag)) return;
-        cur ^= 1;
-        ++iter;
-        // counts only shrink (every iteration merges); the clamps keep a wrong
+    bool hashTies = false, pairNext = false, stop = false;  // the same in every CTA: they follow the cluster counts
+    auto advance = [&](uint32_t next) {
+        // counts only shrink (every iteration merges); the clamp keeps a wrong
         // count from reaching past the buffers
-        const uint32_t next = min(C, ld_acquire(&a.ctl->clusters[iter & 1]));
+        next = min(C, next);
         if ((unsigned long long)(C - next) * 64ull < C) {
             pairNext = hashTies;
             hashTies = true;
@@ -680,87 +755,92 @@ __global__ void __launch_bounds__(kPlocThreads, 3) k_ploc(PlocArgs a)
             pairNext = false;
         }
         C = next;
-        merged = min(a.n - 1, ld_acquire(&a.ctl->merged[iter & 1]));
+    };
+    // ------------------------------------------------------------ grid phase
+    while (C > kTailClusters) {
+        const bool small = C <= kSmallMax;
+        const uint32_t tiles = small ? (C + smallTile - 1) / smallTile : (C + bigTile - 1) / bigTile;
+        // with small tiles their number only falls, and CTAs left without one
+        // take no part any more
+        const uint32_t ctas = small ? min(tiles, gridDim.x) : gridDim.x;
+        if (blockIdx.x >= ctas) break;
+        unsigned long long* flags = a.flags + (size_t)(iter & 1) * a.maxTiles;
+        unsigned long long* nextFlags = a.flags + (size_t)((iter + 1) & 1) * a.maxTiles;
+        const float4* src = cur ? a.clusters[1] : a.clusters[0];
+        float4* dst = cur ? a.clusters[0] : a.clusters[1];
+        // the next iteration's look-back words, as many as it can have tiles (more than now where it is the first
+        // with small ones), shared out over this iteration's tiles
+        const uint32_t most = min(a.maxTiles, max(tiles, (min(C, kSmallMax) + smallTile - 1) / smallTile));
+        const uint32_t share = (most + tiles - 1) / tiles;
+        uint32_t survivors = 0;
+        bool ok = true;
+        for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+            for (uint32_t k = tid; k < share; k += kPlocThreads)
+                if (t * share + k < most) nextFlags[t * share + k] = 0ull;
+            survivors += small ? ploc_tile<R, 1>(a, sh, t, tiles, C, a.n - C, r, pairNext, hashTies, src, dst, flags, ok)
+                               : ploc_tile<R, kPer>(a, sh, t, tiles, C, a.n - C, r, pairNext, hashTies, src, dst,
+                                                    flags, ok);
+        }
+        const uint32_t next = end_iteration(a.ctl, ctas, iter, survivors, !ok, a.error, a.spinLimit, &sNext);
+        if (next == kUnset) {
+            stop = true;
+            break;
+        }
+        cur ^= 1;
+        ++iter;
+        advance(next);
     }
 
     // ------------------------------------------------------------------ tail
     if (blockIdx.x == 0) {
-        const float4* src = cur ? a.clusters[1] : a.clusters[0];
-        for (uint32_t k = tid; k < C; k += kPlocThreads) {
-            sLo[pad(k)] = __ldcg(src + 2ull * k);
-            sHi[pad(k)] = __ldcg(src + 2ull * k + 1);
+        if (!stop) {
+            const float4* src = cur ? a.clusters[1] : a.clusters[0];
+            for (uint32_t k = tid; k < C; k += kPlocThreads) {
+                sh.lo[pad(k)] = __ldcg(src + 2ull * k);
+                sh.hi[pad(k)] = __ldcg(src + 2ull * k + 1);
+            }
+            __syncthreads();
+            while (C > 1) {
+                // fewer clusters per thread while they suffice: the search is one thread's chain
+                const uint32_t next = C > 2 * kPlocThreads ? ploc_tail<R, kPer>(a, sh, C, a.n - C, r, pairNext, hashTies)
+                                      : C > kPlocThreads   ? ploc_tail<R, 2>(a, sh, C, a.n - C, r, pairNext, hashTies)
+                                                           : ploc_tail<R, 1>(a, sh, C, a.n - C, r, pairNext, hashTies);
+                advance(next);
+            }
+            // the root (the last node made) has the first leaf and no parent
+            if (tid == 0) st_relaxed64(a.info + a.n - 2, (unsigned long long)kInvalid << 32);
+            __syncthreads();
+        }
+        if (tid == 0) {
+            __threadfence();
+            st_release(&a.ctl->done, stop ? 2u : 1u);
+        }
+        if (stop) return;
+    } else {
+        if (stop) return;
+        __syncthreads();  // the last count is read
+        if (tid == 0) {
+            uint32_t done, spins = 0;
+            while ((done = ld_acquire(&a.ctl->done)) == 0u) {
+                if (++spins > a.spinLimit) {
+                    atomicOr(a.error, 1u);
+                    done = 2u;
+                    break;
+                }
+                __nanosleep(200);
+            }
+            sNext = done;
         }
         __syncthreads();
-        while (C > 1) {
-            const bool pairs = pairNext;
-            {
-                const uint32_t g0 = kPer * tid;  // C <= kTile: one group per thread
-                if (g0 < C) {
-                    if (pairs)
-                        pair_partners(g0, 0, C, 0, C, sNN);
-                    else
-                        nearest<R>(g0, 0, C, 0, C, r, sLo, sHi, sNN);
-                }
-            }
-            __syncthreads();
-            if (hashTies && !pairs) {
-                const uint32_t g0 = kPer * tid;
-                if (g0 < C) resolve_ties(g0, 0, C, 0, C, r, sLo, sHi, sNN);
-                __syncthreads();
-            }
-            const uint32_t p0 = kPer * tid;
-            const Decision dc = decide(p0, C, 0, sNN);
-            uint32_t total;
-            const uint32_t before = sort::block_scan(__popc(dc.keepMask) | __popc(dc.mergeMask) << 16, sWarp, &total);
-            float4 keepLo[kPer], keepHi[kPer];
-            uint32_t node = merged + (before >> 16);
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                keepLo[q] = keepHi[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (!((dc.keepMask >> q) & 1u)) continue;
-                const uint32_t p = p0 + q;
-                keepLo[q] = sLo[pad(p)];
-                keepHi[q] = sHi[pad(p)];
-                if ((dc.mergeMask >> q) & 1u) {
-                    const uint32_t j = sNN[pad(p)];
-                    if (node < a.n - 1)
-                        merge_pair(a.tmp, node, keepLo[q], keepHi[q], sLo[pad(j)], sHi[pad(j)], keepLo[q], keepHi[q]);
-                    ++node;
-                }
-            }
-            __syncthreads();  // every read of this iteration's clusters is done
-            uint32_t outPos = before & 0xFFFFu;
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                if (!((dc.keepMask >> q) & 1u)) continue;
-                sLo[pad(outPos)] = keepLo[q];
-                sHi[pad(outPos)] = keepHi[q];
-                ++outPos;
-            }
-            merged += total >> 16;
-            const uint32_t next = total & 0xFFFFu;
-            if ((unsigned long long)(C - next) * 64ull < C) {
-                pairNext = hashTies;
-                hashTies = true;
-            } else {
-                pairNext = false;
-            }
-            C = next;
-            __syncthreads();
-        }
-        // the root (the last node made) has the first leaf and no parent
-        if (tid == 0 && merged > 0)
-            st_relaxed64(a.info + merged - 1, (unsigned long long)kInvalid << 32);
+        if (sNext != 1u) return;
     }
-    if (!grid_barrier(a.ctl, a.error, a.spinLimit, &sFlag)) return;
 
     // ------------------------------------------------------------- placement
     place_all(a);
 }
 
 // The cooperative launch of k_ploc<R> with as many CTAs as can be resident
-// (at most kMaxCtasPerSm per multiprocessor, at most one per first-iteration
-// tile).
+// (at most kMaxCtasPerSm per multiprocessor, at most one per tile).
 template <int R>
 mlbvh_status launch_ploc(PlocArgs& a, uint32_t firstTiles, cudaStream_t stream)
 {
@@ -828,7 +908,9 @@ mlbvh_status build_ploc(const mlbvh_triangle* dTris, uint32_t n, uint32_t option
 
     ProfileEvents ev = take_profile_events();
     if (ev.start) cudaEventRecord(ev.start, stream);
-    const uint32_t firstTiles = (n + (kTile - 2u * radius) - 1) / (kTile - 2u * radius);
+    const uint32_t few = std::min(n, kSmallMax), smallTile = kPlocThreads - 2u * radius, bigTile = kTile - 2u * radius;
+    const uint32_t firstTiles = std::max(n > kSmallMax ? (n + bigTile - 1) / bigTile : 0u,
+                                         (few + smallTile - 1) / smallTile);
     switch (radius) {
         case 4: st = launch_ploc<4>(a, firstTiles, stream); break;
         case 8: st = launch_ploc<8>(a, firstTiles, stream); break;
