@@ -307,14 +307,67 @@ __device__ __forceinline__ void nearest_fixed(uint32_t p0, uint32_t first, uint3
     }
 }
 
+// nearest_fixed for groups at the ends of the clusters, whose windows are cut
+// off: the same unrolled loops, every candidate's position tested.
 template <int R, int kPer>
-__device__ __forceinline__ void nearest(uint32_t p0, uint32_t first, uint32_t end, uint32_t base, uint32_t staged,
-                                        int r, const float4* sLo, const float4* sHi, uint32_t* sNN)
+__device__ __forceinline__ void nearest_edge(uint32_t p0, uint32_t first, uint32_t end, uint32_t base,
+                                             uint32_t staged, const float4* sLo, const float4* sHi, uint32_t* sNN)
 {
-    if (R > 0 && p0 >= base + R && p0 + kPer - 1 + R < staged)
-        nearest_fixed<R, kPer>(p0, first, end, base, sLo, sHi, sNN);
-    else
-        nearest_group<kPer>(p0, first, end, base, staged, r, sLo, sHi, sNN);
+    f3 plo[kPer], phi[kPer];
+    uint32_t bestA[kPer], bestJ[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t p = min(p0 + q, staged - 1);
+        plo[q] = xyz(sLo[pad(p - base)]);
+        phi[q] = xyz(sHi[pad(p - base)]);
+        bestA[q] = 0xFFFFFFFFu;
+        bestJ[q] = 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * R + kPer; ++k) {
+        const int j = (int)p0 + k - R;
+        const bool there = j >= (int)base && j < (int)staged;
+        const uint32_t at = (uint32_t)min(max(j, (int)base), (int)staged - 1);
+        const f3 jlo = xyz(sLo[pad(at - base)]), jhi = xyz(sHi[pad(at - base)]);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int d = k - R - q;
+            if (d == 0 || d < -R || d > R) continue;
+            const uint32_t a = area_key(plo[q], phi[q], jlo, jhi);
+            if (there && a < bestA[q]) {
+                bestA[q] = a;
+                bestJ[q] = (uint32_t)j;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t p = p0 + q;
+        if (p >= first && p < end) sNN[pad(p - base)] = bestJ[q];
+    }
+}
+
+// The nearest neighbours of a thread's group; `in` is false for threads without
+// one. Every thread of the warp calls it: a warp with a group at an end takes
+// the edge loops as a whole instead of both in turn (a CTA at an end, and the
+// tail, took 4.8 us for its search with a plain loop there).
+template <int R, int kPer>
+__device__ __forceinline__ void nearest(bool in, uint32_t p0, uint32_t first, uint32_t end, uint32_t base,
+                                        uint32_t staged, int r, const float4* sLo, const float4* sHi, uint32_t* sNN)
+{
+    const bool edge = in && !(p0 >= base + R && p0 + kPer - 1 + R < staged);
+    if constexpr (R > 0 && R <= 16) {
+        if (__any_sync(0xffffffffu, edge)) {
+            if (in) nearest_edge<R, kPer>(p0, first, end, base, staged, sLo, sHi, sNN);
+        } else if (in) {
+            nearest_fixed<R, kPer>(p0, first, end, base, sLo, sHi, sNN);
+        }
+    } else if (in) {  // 32: the edge loops spill
+        if (R > 0 && !edge)
+            nearest_fixed<R, kPer>(p0, first, end, base, sLo, sHi, sNN);
+        else
+            nearest_group<kPer>(p0, first, end, base, staged, r, sLo, sHi, sNN);
+    }
 }
 
 // A pairing iteration: position 2k's neighbour is 2k + 1 and the other way
@@ -632,12 +685,10 @@ __device__ __forceinline__ uint32_t ploc_tile(const PlocArgs& a, const PlocShare
     __syncthreads();
     const uint32_t nnFirst = s > (uint32_t)r ? s - r : 0u, nnEnd = min(C, e + r);
     const uint32_t g0 = nnFirst + kPer * tid;  // nnEnd - nnFirst <= kPlocThreads * kPer: one group per thread
-    if (g0 < nnEnd) {
-        if (pairs)
-            pair_partners<kPer>(g0, nnFirst, nnEnd, base, C, sh.nn);
-        else
-            nearest<R, kPer>(g0, nnFirst, nnEnd, base, stagedEnd, r, sh.lo, sh.hi, sh.nn);
-    }
+    if (!pairs)
+        nearest<R, kPer>(g0 < nnEnd, g0, nnFirst, nnEnd, base, stagedEnd, r, sh.lo, sh.hi, sh.nn);
+    else if (g0 < nnEnd)
+        pair_partners<kPer>(g0, nnFirst, nnEnd, base, C, sh.nn);
     __syncthreads();
     if (hashTies && !pairs) {  // uniform over the grid
         if (g0 < nnEnd) resolve_ties<kPer>(g0, nnFirst, nnEnd, base, stagedEnd, r, sh.lo, sh.hi, sh.nn);
@@ -684,12 +735,10 @@ __device__ __forceinline__ uint32_t ploc_tail(const PlocArgs& a, const PlocShare
                                               int r, bool pairs, bool hashTies)
 {
     const uint32_t g0 = kPer * threadIdx.x;
-    if (g0 < C) {
-        if (pairs)
-            pair_partners<kPer>(g0, 0, C, 0, C, sh.nn);
-        else
-            nearest<R, kPer>(g0, 0, C, 0, C, r, sh.lo, sh.hi, sh.nn);
-    }
+    if (!pairs)
+        nearest<R, kPer>(g0 < C, g0, 0, C, 0, C, r, sh.lo, sh.hi, sh.nn);
+    else if (g0 < C)
+        pair_partners<kPer>(g0, 0, C, 0, C, sh.nn);
     __syncthreads();
     if (hashTies && !pairs) {
         if (g0 < C) resolve_ties<kPer>(g0, 0, C, 0, C, r, sh.lo, sh.hi, sh.nn);
