@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "capi_internal.h"
+#include "chain.cuh"
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(kPlanThreads)
 {
     __shared__ uint32_t s_warp[33];
     __shared__ uint32_t s_bad;
+    chain_begin();
     if (threadIdx.x == 0) s_bad = (__ldg(off) != 0u || __ldg(off + nMeshes) != n) ? 1u : 0u;
     if (threadIdx.x < 8) header[threadIdx.x] = 0u;  // error word and tile tickets
     if (threadIdx.x == kHdrQueue) header[kHdrQueue] = 0u;
@@ -259,6 +261,7 @@ __global__ void __launch_bounds__(kTileThreads)
                    const uint32_t* __restrict__ tileStart, uint32_t* __restrict__ bounds,
                    uint32_t* __restrict__ zeroBegin, size_t zeroWords)
 {
+    chain_begin();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < zeroWords; i += (size_t)gridDim.x * blockDim.x)
         zeroBegin[i] = 0u;
     TileWork w;
@@ -324,6 +327,7 @@ __global__ void __launch_bounds__(kTileThreads)
     constexpr uint32_t kMask = (uint32_t)kBins - 1u;
     __shared__ uint32_t s_hist[kPasses * kBins];
     __shared__ __align__(16) float s_tri[kStageTris * 9];
+    chain_begin();
     TileWork w;
     if (!tile_work(off, tileStart, nMeshes, blockIdx.x, w)) return;
     for (int i = threadIdx.x; i < kPasses * kBins; i += kTileThreads) s_hist[i] = 0u;
@@ -552,11 +556,11 @@ mlbvh_status launch_build(const mlbvh_batch& B, const BatchLayout& L, cudaStream
     k_batch_plan<<<1, kPlanThreads, 0, stream>>>(off, nm, n, header, tileStart, bounds);
     MLBVH_CHECK_LAUNCH("k_batch_plan");
     const size_t zeroWords = (L.zeroEnd - L.histogram) / 4;
-    k_batch_bounds<<<L.maxTiles, kTileThreads, 0, stream>>>(tris, n, off, nm, tileStart, bounds, hist, zeroWords);
+    launch_chained(k_batch_bounds, L.maxTiles, kTileThreads, 0, stream, tris, n, off, nm, tileStart, bounds, hist,
+                   zeroWords);
     MLBVH_CHECK_LAUNCH("k_batch_bounds");
-    k_batch_keys<kBits><<<L.maxTiles, kTileThreads, 0, stream>>>(tris, n, B.buildOption, off, nm, tileStart, bounds,
-                                                                 keysA, hist, handoff, B.dMeshAABBs,
-                                                                 header + kHdrTreeFlags);
+    launch_chained(k_batch_keys<kBits>, L.maxTiles, kTileThreads, 0, stream, tris, n, B.buildOption, off, nm, tileStart,
+                   bounds, keysA, hist, handoff, B.dMeshAABBs, header + kHdrTreeFlags);
     MLBVH_CHECK_LAUNCH("k_batch_keys");
     uint32_t* kin = keysA;
     uint32_t* vin = valsA;
@@ -565,12 +569,11 @@ mlbvh_status launch_build(const mlbvh_batch& B, const BatchLayout& L, cudaStream
         uint32_t* vout = (pass % 2 == 0) ? valsB : valsA;
         const sort::MeshSegments segs{off, tileStart, nm, hist + (size_t)pass * kBins, (uint32_t)(kPasses * kBins)};
         uint32_t* lb = lookback + (size_t)pass * L.maxTiles * kBins;
-        if (pass == 0)
-            sort::k_onesweep<kBits, true><<<L.maxTiles, sort::kThreads, S::kSmemBytes, stream>>>(
-                kin, kout, nullptr, vout, kBits * pass, segs, lb, header + kHdrTickets + pass, header, spinLimit);
-        else
-            sort::k_onesweep<kBits, false><<<L.maxTiles, sort::kThreads, S::kSmemBytes, stream>>>(
-                kin, kout, vin, vout, kBits * pass, segs, lb, header + kHdrTickets + pass, header, spinLimit);
+        auto kernel = pass == 0 ? sort::k_onesweep<kBits, true, sort::MeshSegments>
+                                : sort::k_onesweep<kBits, false, sort::MeshSegments>;
+        launch_chained(kernel, L.maxTiles, sort::kThreads, S::kSmemBytes, stream, kin, kout,
+                       pass == 0 ? nullptr : vin, vout, kBits * pass, segs, lb, header + kHdrTickets + pass, header,
+                       spinLimit);
         MLBVH_CHECK_LAUNCH("k_onesweep");
         kin = kout;
         vin = vout;

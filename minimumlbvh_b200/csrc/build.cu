@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "capi_internal.h"
+#include "chain.cuh"
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(kBoundsThreads)
     k_scene_bounds(const float* __restrict__ tris, uint32_t n, float* __restrict__ partials,
                    uint32_t* __restrict__ zeroBegin, size_t zeroWords)
 {
+    chain_begin();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t nthreads = (size_t)gridDim.x * blockDim.x;
     for (size_t i = tid; i < zeroWords; i += nthreads) zeroBegin[i] = 0u;
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(kKeysThreads)
     __shared__ float s_scene[6];
     __shared__ uint32_t s_hist[4][256];
     __shared__ float4 s_tri[kKeysThreads / 32][72];  // 32 triangles of 9 floats per warp
+    chain_begin();
 
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t chunks = (n + 31) / 32, warps = gridDim.x * (kKeysThreads / 32);
@@ -289,8 +292,8 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
     k_scene_bounds<<<boundsBlocks, kBoundsThreads, 0, stream>>>(tris, n, partials, header, zeroWords);
     MLBVH_CHECK_LAUNCH("k_scene_bounds");
     const int keysBlocks = (int)std::max<uint32_t>(1, std::min<uint32_t>((n + 4 * kKeysThreads - 1) / (4 * kKeysThreads), 4u * sms));
-    k_keys<<<keysBlocks, kKeysThreads, 0, stream>>>(tris, n, option, partials, boundsBlocks, keysA, hist, handoff,
-                                                    dScene, header + kHdrTreeFlags);
+    launch_chained(k_keys, keysBlocks, kKeysThreads, 0, stream, tris, n, option, partials, boundsBlocks, keysA, hist,
+                   handoff, dScene, header + kHdrTreeFlags);
     MLBVH_CHECK_LAUNCH("k_keys");
 
     uint32_t* kin = keysA;
@@ -305,9 +308,8 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
         auto kernel = few ? (pass == 0 ? sort::k_onesweep<8, true, Seg, sort::kFewItems>
                                        : sort::k_onesweep<8, false, Seg, sort::kFewItems>)
                           : (pass == 0 ? sort::k_onesweep<8, true, Seg> : sort::k_onesweep<8, false, Seg>);
-        kernel<<<L.tiles, sort::kThreads, smem, stream>>>(kin, kout, pass == 0 ? nullptr : vin, vout, 8 * pass, seg,
-                                                          lookback + (size_t)pass * L.tiles * 256, header + 1 + pass,
-                                                          header, spinLimit);
+        launch_chained(kernel, L.tiles, sort::kThreads, smem, stream, kin, kout, pass == 0 ? nullptr : vin, vout,
+                       8 * pass, seg, lookback + (size_t)pass * L.tiles * 256, header + 1 + pass, header, spinLimit);
         MLBVH_CHECK_LAUNCH("k_onesweep");
         kin = kout;
         vin = vout;

@@ -22,6 +22,8 @@
 
 #include <cstdint>
 
+#include "chain.cuh"
+
 namespace mlbvh {
 namespace sort {
 
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
     __shared__ uint32_t s_scan[kWarps];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    chain_begin();
     if (tid == 0) {
         const uint32_t t = atomicAdd(tileCounter, 1u);
         Segment sg;

@@ -56,6 +56,7 @@
 #include <algorithm>
 
 #include "capi_internal.h"
+#include "chain.cuh"
 #include "../../include/mlbvh_device.cuh"
 #include "climb.cuh"
 #include "onesweep.cuh"
@@ -636,6 +637,7 @@ __global__ void __launch_bounds__(kInitThreads)
                 float4* __restrict__ clusters, unsigned long long* __restrict__ flags, uint32_t nFlags,
                 PlocControl* __restrict__ ctl, unsigned long long* __restrict__ info)
 {
+    chain_begin();
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t i = g; i < nFlags; i += stride) flags[i] = 0ull;
@@ -951,8 +953,8 @@ mlbvh_status build_ploc(const mlbvh_triangle* dTris, uint32_t n, uint32_t option
 
     const int sms = device_sm_count();
     const int initBlocks = std::max(1, std::min<int>((n + kInitThreads - 1) / kInitThreads, 8 * sms));
-    k_ploc_init<<<initBlocks, kInitThreads, 0, stream>>>(reinterpret_cast<const float*>(dTris), sl.indices, n,
-                                                         a.clusters[0], a.flags, 2 * L.maxTiles, a.ctl, a.info);
+    launch_chained(k_ploc_init, initBlocks, kInitThreads, 0, stream, reinterpret_cast<const float*>(dTris), sl.indices, n,
+                   a.clusters[0], a.flags, 2 * L.maxTiles, a.ctl, a.info);
     MLBVH_CHECK_LAUNCH("k_ploc_init");
 
     ProfileEvents ev = take_profile_events();

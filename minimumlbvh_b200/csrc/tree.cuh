@@ -51,6 +51,7 @@
 
 #include "../../include/mlbvh.h"
 #include "../../include/mlbvh_device.cuh"
+#include "chain.cuh"
 #include "climb.cuh"
 
 namespace mlbvh {
@@ -251,6 +252,7 @@ __device__ __forceinline__ void reduce_block(const Level& from, const Level& to,
 // One warp per group; the last group of a super to finish reduces it.
 static __global__ void __launch_bounds__(128) k_tree_groups(Scratch sc)
 {
+    chain_begin();
     const uint32_t groups = (sc.nTiles + 31) / 32, g = (blockIdx.x * 128 + threadIdx.x) >> 5;
     if (g >= groups || (__ldcg(sc.flags) & (kNaN | kSkip))) return;
     reduce_block(sc.level[0], sc.level[1], sc.nTiles, g);
@@ -296,6 +298,7 @@ __global__ void __launch_bounds__(kTile, kTileCtas)
     __shared__ uint32_t s_nWide, s_record0;
     __shared__ Box s_warpBox[kWarps], s_before[kWarps], s_after[kWarps];
     __shared__ uint32_t s_mesh[Trees::kMany ? kTile : 1];
+    chain_begin();
     if (__ldcg(sc.flags) & (kNaN | kSkip)) return;  // the whole CTA: set before this launch
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = sc.n;
@@ -753,6 +756,7 @@ __global__ void __launch_bounds__(kCrossThreads)
                  mlbvh_node_index* __restrict__ roots, uint32_t* __restrict__ handoff, Scratch sc)
 {
     __shared__ uint32_t s_far[kCrossNodes], s_nFar;
+    chain_begin();
     const uint32_t thread = blockIdx.x * kCrossThreads + threadIdx.x, threads = gridDim.x * kCrossThreads;
     const uint32_t flags = __ldcg(sc.flags);
     if (flags & kSkip) return;
@@ -882,21 +886,23 @@ __global__ void __launch_bounds__(kCrossThreads)
     }
 }
 
-// Launches the kernels. handoff: n words of ~0 (the climb's).
+// Launches the kernels after the sort's (chain.cuh). handoff: n words of ~0 (the climb's).
 template <class Trees>
 inline mlbvh_status launch(const float* tris, const Trees& trees, const uint32_t* keys, const uint32_t* idx,
                            mlbvh_internal_node* nodes, mlbvh_node_index* roots, uint8_t* deltasOut, uint32_t* handoff,
                            const Scratch& sc, int sms, cudaStream_t stream)
 {
     const uint32_t tileBlocks = std::min<uint32_t>(sc.nTiles, kTileCtas * (uint32_t)sms);
-    k_tree_tiles<<<tileBlocks, kTile, 0, stream>>>(tris, trees, keys, idx, nodes, roots, deltasOut, sc);
+    launch_chained(k_tree_tiles<Trees>, tileBlocks, kTile, 0, stream, tris, trees, keys, idx, nodes, roots, deltasOut,
+                   sc);
     MLBVH_CHECK_LAUNCH("k_tree_tiles");
     if (sc.nTiles > 32) {
-        k_tree_groups<<<(up32(sc.nTiles) + 3) / 4, 128, 0, stream>>>(sc);
+        launch_chained(k_tree_groups, (up32(sc.nTiles) + 3) / 4, 128, 0, stream, sc);
         MLBVH_CHECK_LAUNCH("k_tree_groups");
     }
     const uint32_t blocks = std::min<uint32_t>(sc.n / 24 / kCrossNodes + 1, 32u * (uint32_t)sms);
-    k_tree_cross<<<blocks, kCrossThreads, 0, stream>>>(tris, trees, keys, idx, nodes, roots, handoff, sc);
+    launch_chained(k_tree_cross<Trees>, blocks, kCrossThreads, 0, stream, tris, trees, keys, idx, nodes, roots, handoff,
+                   sc);
     MLBVH_CHECK_LAUNCH("k_tree_cross");
     return MLBVH_OK;
 }
