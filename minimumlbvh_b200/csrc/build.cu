@@ -4,7 +4,8 @@
 // Replaces BVHGPUBuilder::build (minimum_lbvh.h:783-871), its kernels
 // (minimum_lbvh.cu:38-120) and OnesweepSort (tinyhiponesweep.h:592-668).
 //
-// Launch chain on one stream (no host synchronisation):
+// Launch chain on one stream (no host synchronisation; up to 4,096 triangles
+// k_small_sort stands for the first three rows):
 //   k_scene_bounds   per-CTA partial bounds of all vertices; zeroes the
 //                    sort's counters, histograms and look-back words
 //   k_keys           reduces the partial bounds, writes the 32-bit Morton key
@@ -44,6 +45,14 @@ constexpr int kKeysThreads = 256;
 constexpr uint32_t kFewMax = 3 * 148 * sort::kThreads * sort::kFewItems;
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
 constexpr int kHdrTreeFlags = 5;  // header word of tree::Scratch::flags; the record count follows
+
+// Arrays up to this size take one CTA from the triangles to the sorted keys
+// (k_small_sort) instead of the bounds, key and sort kernels, whose launches and
+// look-backs cost more than their work. Whole builds, one CTA / chain: 100
+// triangles 21 / 36 us, 1,000 24 / 35, 2,000 29 / 38, 4,000 38 / 40; 6,000 52 /
+// 42.
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallMax = 4 * kSmallThreads;
 
 // Scratch layout of one build (offsets from the caller's dScratch). The
 // leading region [header, partials) is zeroed by k_scene_bounds on every build.
@@ -258,6 +267,205 @@ __global__ void __launch_bounds__(kKeysThreads)
     }
 }
 
+// The chain up to the sorted keys for few triangles, in one CTA: scene bounds
+// (k_scene_bounds), keys (triangle_key) and four stable passes of 8 bits in
+// shared memory, each a warp multisplit over warps of kPer x 32 consecutive
+// keys. The same keys, order and words as the kernels above: fminf and fmaxf
+// give the same bounds in any order.
+template <int kPer>
+struct SmallShared {
+    uint32_t count[32][256];   // per warp and digit, then the warps' offsets within the digit
+    uint32_t part[4][256];     // the same for the four groups of eight warps
+    uint32_t start[256];       // first position of each digit
+    uint32_t keys[kSmallThreads * kPer], vals[kSmallThreads * kPer];
+    float box[32][6];
+    uint32_t scan[8];
+};
+template <int kPer>
+__global__ void __launch_bounds__(kSmallThreads)
+    k_small_sort(const float* __restrict__ tris, uint32_t n, uint32_t option, uint32_t* __restrict__ header,
+                 uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut, uint32_t* __restrict__ handoff,
+                 mlbvh_aabb* __restrict__ sceneOut)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SmallShared<kPer>& sh = *reinterpret_cast<SmallShared<kPer>*>(smem);
+    chain_begin();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < 8) header[tid] = 0u;
+    // ---- bounds, as k_scene_bounds
+    float lo[3] = {kFltMax, kFltMax, kFltMax}, hi[3] = {-kFltMax, -kFltMax, -kFltMax};
+    const uint32_t nFloats = n * 9, nGroups = nFloats / 12;
+    const float4* t4 = reinterpret_cast<const float4*>(tris);
+    for (uint32_t g = tid; g < nGroups; g += kSmallThreads) {
+        const float4 a = __ldg(t4 + 3 * g), b = __ldg(t4 + 3 * g + 1), c = __ldg(t4 + 3 * g + 2);
+        lo[0] = fminf(lo[0], fminf(fminf(a.x, a.w), fminf(b.z, c.y)));
+        hi[0] = fmaxf(hi[0], fmaxf(fmaxf(a.x, a.w), fmaxf(b.z, c.y)));
+        lo[1] = fminf(lo[1], fminf(fminf(a.y, b.x), fminf(b.w, c.z)));
+        hi[1] = fmaxf(hi[1], fmaxf(fmaxf(a.y, b.x), fmaxf(b.w, c.z)));
+        lo[2] = fminf(lo[2], fminf(fminf(a.z, b.y), fminf(c.x, c.w)));
+        hi[2] = fmaxf(hi[2], fmaxf(fmaxf(a.z, b.y), fmaxf(c.x, c.w)));
+    }
+    for (uint32_t j = nGroups * 12 + tid; j < nFloats; j += kSmallThreads) {
+        const float v = __ldg(tris + j);
+        const uint32_t ax = j % 3;
+#pragma unroll
+        for (uint32_t a = 0; a < 3; ++a)
+            if (ax == a) {
+                lo[a] = fminf(lo[a], v);
+                hi[a] = fmaxf(hi[a], v);
+            }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            sh.box[warp][a] = lo[a];
+            sh.box[warp][3 + a] = hi[a];
+        }
+    __syncthreads();  // also orders the header's zeros before treeFlags below
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = sh.box[lane][a];
+        hi[a] = sh.box[lane][3 + a];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
+    if (sceneOut && tid == 0) {
+        float* out = reinterpret_cast<float*>(sceneOut);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            out[a] = lo[a];
+            out[3 + a] = hi[a];
+        }
+    }
+    // ---- keys
+    const f3 lower = mk(lo[0], lo[1], lo[2]), upper = mk(hi[0], hi[1], hi[2]);
+    uint32_t key[kPer], val[kPer], rank[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const uint32_t i = warp * (32 * kPer) + k * 32 + lane;
+        val[k] = i;
+        key[k] = 0xFFFFFFFFu;
+        if (i < n) {
+            float t[9];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) t[j] = __ldg(tris + 9 * i + j);
+            key[k] = triangle_key(t, option, lower, upper, header + kHdrTreeFlags);
+            handoff[i] = 0xFFFFFFFFu;
+        }
+    }
+    // ---- four passes
+    for (int shift = 0; shift < 32; shift += 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sh.count[warp][32 * j + lane] = 0u;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t i = warp * (32 * kPer) + k * 32 + lane;
+            const uint32_t d = (key[k] >> shift) & 255u;
+            uint32_t peers = __ballot_sync(0xffffffffu, i < n);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const uint32_t bit = (d >> b) & 1u;
+                const uint32_t m = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? m : ~m;
+            }
+            const uint32_t before = sh.count[warp][d];
+            rank[k] = before + __popc(peers & ((1u << lane) - 1u));
+            __syncwarp();
+            if (i < n && lane == __ffs(peers) - 1) sh.count[warp][d] = before + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        {  // eight warps' counts of one digit per thread
+            const uint32_t d = tid & 255u, group = tid >> 8;
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < 8; ++w) {
+                const uint32_t x = sh.count[8 * group + w][d];
+                sh.count[8 * group + w][d] = c;
+                c += x;
+            }
+            sh.part[group][d] = c;
+        }
+        __syncthreads();
+        uint32_t total = 0, inc = 0;
+        if (tid < 256) {  // the digits' starts
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g) {
+                const uint32_t x = sh.part[g][tid];
+                sh.part[g][tid] = c;
+                c += x;
+            }
+            total = inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if ((int)lane >= o) inc += y;
+            }
+            if (lane == 31) sh.scan[warp] = inc;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            for (uint32_t w = 0; w < warp; ++w) inc += sh.scan[w];
+            sh.start[tid] = inc - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t i = warp * (32 * kPer) + k * 32 + lane;
+            if (i < n) {
+                const uint32_t d = (key[k] >> shift) & 255u;
+                const uint32_t pos = sh.start[d] + sh.part[warp >> 3][d] + sh.count[warp][d] + rank[k];
+                sh.keys[pos] = key[k];
+                sh.vals[pos] = val[k];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t i = warp * (32 * kPer) + k * 32 + lane;
+            if (i < n) {
+                key[k] = sh.keys[i];
+                val[k] = sh.vals[i];
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const uint32_t i = warp * (32 * kPer) + k * 32 + lane;
+        if (i < n) {
+            keysOut[i] = key[k];
+            valsOut[i] = val[k];
+        }
+    }
+}
+
+template <int kPer>
+mlbvh_status launch_small_sort(const float* tris, uint32_t n, uint32_t option, uint32_t* header, uint32_t* keys,
+                               uint32_t* vals, uint32_t* handoff, mlbvh_aabb* scene, cudaStream_t stream)
+{
+    constexpr int smem = (int)sizeof(SmallShared<kPer>);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_small_sort<kPer>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return fail(MLBVH_ERR_LAUNCH, cudaGetErrorString(e));
+    k_small_sort<kPer><<<1, kSmallThreads, smem, stream>>>(tris, n, option, header, keys, vals, handoff, scene);
+    MLBVH_CHECK_LAUNCH("k_small_sort");
+    return MLBVH_OK;
+}
+
 }  // namespace
 
 size_t build_scratch_bytes(uint32_t n) { return build_layout(n).total; }
@@ -281,6 +489,21 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
     uint32_t* keysFinal = dKeysOut ? dKeysOut : keysA;
     uint32_t* valsFinal = dIdxOut ? dIdxOut : valsA;
     const float* tris = reinterpret_cast<const float*>(dTris);
+
+    out->keys = keysFinal;
+    out->indices = valsFinal;
+    out->error = header;
+    out->handoff = handoff;
+    // after the last pass its inputs are free
+    out->tree = tree::place(n, s + L.summary, reinterpret_cast<uint32_t*>(s + L.treeCounts), header + kHdrTreeFlags,
+                               keysB);
+    out->spinLimit = spinLimit;
+    if (n <= kSmallMax)
+        return n <= kSmallThreads ? launch_small_sort<1>(tris, n, option, header, keysFinal, valsFinal, handoff, dScene,
+                                                         stream)
+               : n <= 2 * kSmallThreads
+                   ? launch_small_sort<2>(tris, n, option, header, keysFinal, valsFinal, handoff, dScene, stream)
+                   : launch_small_sort<4>(tris, n, option, header, keysFinal, valsFinal, handoff, dScene, stream);
 
     const int sms = device_sm_count();
     const size_t zeroWords = (L.partials - L.header) / 4;
@@ -314,14 +537,6 @@ mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t optio
         kin = kout;
         vin = vout;
     }
-    out->keys = keysFinal;
-    out->indices = valsFinal;
-    out->error = header;
-    out->handoff = handoff;
-    // after four passes the last pass's inputs are free
-    out->tree = tree::place(n, s + L.summary, reinterpret_cast<uint32_t*>(s + L.treeCounts), header + kHdrTreeFlags,
-                               keysB);
-    out->spinLimit = spinLimit;
     return MLBVH_OK;
 }
 
