@@ -398,7 +398,8 @@ constexpr int kBatchReplayDepth = 16;  // stack entries per lane of the replay w
 constexpr int kBatchNodeSteps = 5;
 
 template <bool kAny, bool kReplay>
-__global__ void __launch_bounds__(512)
+// 64 registers (1,074 us against 1,092 at the 68 it takes without the bound)
+__global__ void __launch_bounds__(512, 2)
     k_batch_trace(const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ roots,
                   const float* __restrict__ tris, const uint32_t* __restrict__ triOff,
                   const float4* __restrict__ rays, const uint32_t* __restrict__ rayOff, uint32_t nMeshes,
