@@ -102,15 +102,3 @@ def test_adjoint_full_config(scene):
     host = O.diff_adjoint(out, tris, cam.as_array(), w, h, spp, 3, alb, em, grad_image)
     sel = pick(host, seed=9)
     np.testing.assert_allclose(gpu[sel], host[sel], rtol=REL_TOL)
-
-
-@pytest.mark.parametrize("w,h,spp", [(211, 101, 1), (160, 140, 5), (150, 80, 65), (33, 9, 130), (1, 1, 200)])
-def test_diff_render_units_and_pixel_ranges(scene, w, h, spp):
-    """Warps that take several pixels, units of 64 samples that hold many
-    pixels or a part of one, and a single pixel, bit for bit."""
-    import torch
-    tris, alb, em, b, t, out = scene
-    cam = camera(w, h)
-    img = torch.empty(w * h, dtype=torch.float32, device="cuda")
-    mb.pt_diff_render(img, (w, h), cam, b, t, G.dev(alb), G.dev(em), spp, 2)
-    np.testing.assert_array_equal(G.host(img), O.diff_render(out, tris, cam.as_array(), w, h, spp, 2, alb, em))
