@@ -980,11 +980,11 @@ def profile_case(name, dev):
       trace_wide_closest      4M soup, 1M camera rays closest-hit over the
                               quantised 4-wide slots (k_trace_wide)
       camera_replay_lbvh/_ploc 4M soup, the same camera rays closest-hit on the
-                              replay walk (k_trace) over the LBVH / the PLOC tree
+                              replay walk (k_trace_replay) over the LBVH / the PLOC tree
       batch_trace             48 meshes of the batched workload (64..262,144
                               triangles, 4,096..1M rays each): k_batch_trace
       pt                      heightfield + icospheres, one 512x512 path-tracing
-                              pass (k_pt, stack-free walk)
+                              pass (k_pt)
       adjoint                 the differentiation workload (512x512, 64 spp, 3
                               bounces): k_pt_diff_render, k_pt_diff_adjoint"""
     import torch
