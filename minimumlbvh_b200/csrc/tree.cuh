@@ -42,7 +42,7 @@
 // 256 meshes of 64-65,536 triangles 180 against 264 us. k_tree_tiles executes
 // about 1,000 instructions per 32 leaves at half the issue rate and reads 534
 // MB (64-byte DRAM granules for 36-byte triangles in random order), so it is
-// bound by issue and barriers, at 40 % of the DRAM rate; 4 CTAs per SM because
+// bound by issue and barriers, at 40 % of the DRAM rate; few CTAs per SM because
 // 5 to 7 (without the copies ahead) left the triangle loads no L1: 275 to 389
 // us. k_tree_cross is a chain of 5 to 15 dependent L2 loads.
 #pragma once
@@ -64,7 +64,10 @@ constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kStride = kTile + 2;  // staged words: 4 kStride = 8 mod 32, so a row's store reads distinct banks
 constexpr uint32_t kNaN = 1u, kFull = 2u;  // flag bits: climb this build instead
 constexpr uint32_t kSkip = 4u;             // flag bit: build nothing (bad batch offsets)
-constexpr int kTileCtas = 4;   // resident CTAs per SM of k_tree_tiles (45 KB of shared memory and 64 registers a thread)
+// Resident CTAs per SM of k_tree_tiles: 3 leave a thread 75-78 registers; at 4
+// (64) whole builds took 60.4 us instead of 58.3 at 65k triangles, 86.5 instead
+// of 83.3 at 213k, 181 instead of 179 at 1M and the same 530 at 4M.
+constexpr int kTileCtas = 3;
 constexpr int kCrossThreads = 128;
 constexpr uint32_t kCrossNodes = 64;  // records per CTA and round of k_tree_cross
 constexpr uint32_t kCrossLanes = 8;  // lanes per crossing node
