@@ -756,7 +756,8 @@ template <class Trees>
 __global__ void __launch_bounds__(kCrossThreads)
     k_tree_cross(const float* __restrict__ tris, Trees trees, const uint32_t* __restrict__ keys,
                  const uint32_t* __restrict__ idx, mlbvh_internal_node* __restrict__ nodes,
-                 mlbvh_node_index* __restrict__ roots, uint32_t* __restrict__ handoff, Scratch sc)
+                 mlbvh_node_index* __restrict__ roots, uint8_t* __restrict__ deltasOut, uint32_t* __restrict__ handoff,
+                 Scratch sc)
 {
     __shared__ uint32_t s_far[kCrossNodes], s_nFar;
     chain_begin();
@@ -767,6 +768,8 @@ __global__ void __launch_bounds__(kCrossThreads)
         for (uint32_t g = thread; g < sc.n; g += threads) {
             const Segment seg = trees.of(g);
             const uint32_t tri = idx[g], len = seg.end - seg.start;
+            // k_tree_tiles leaves before its deltas where a centroid is NaN
+            if (deltasOut && g + 1 < seg.end) deltasOut[g] = (uint8_t)delta_at(keys, g);
             if (tri >= len) continue;  // a bounded wait of the sort gave up (error word set)
             f3 lo, hi;
             leaf_box(tris + 9 * (size_t)seg.start, len, tri, lo, hi);
@@ -904,8 +907,8 @@ inline mlbvh_status launch(const float* tris, const Trees& trees, const uint32_t
         MLBVH_CHECK_LAUNCH("k_tree_groups");
     }
     const uint32_t blocks = std::min<uint32_t>(sc.n / 24 / kCrossNodes + 1, 32u * (uint32_t)sms);
-    launch_chained(k_tree_cross<Trees>, blocks, kCrossThreads, 0, stream, tris, trees, keys, idx, nodes, roots, handoff,
-                   sc);
+    launch_chained(k_tree_cross<Trees>, blocks, kCrossThreads, 0, stream, tris, trees, keys, idx, nodes, roots,
+                   deltasOut, handoff, sc);
     MLBVH_CHECK_LAUNCH("k_tree_cross");
     return MLBVH_OK;
 }
