@@ -172,8 +172,10 @@ MLBVH_API const char* mlbvh_last_error_string(void);
  *
  * dInternals receives nTriangles-1 nodes, *dRootNode the root (a leaf when
  * nTriangles == 1). dSceneAABB may be NULL. dScratch must hold
- * mlbvh_build_scratch_bytes(nTriangles) bytes; its contents need no
- * initialisation and must not be shared by builds in flight at the same time.
+ * mlbvh_build_scratch_bytes(nTriangles) bytes, a size that never falls as
+ * nTriangles grows (scratch for the largest scene serves every smaller one);
+ * its contents need no initialisation and must not be shared by builds in
+ * flight at the same time.
  * 1 <= nTriangles < 2^30. */
 MLBVH_API size_t mlbvh_build_scratch_bytes(uint32_t nTriangles);
 MLBVH_API mlbvh_status mlbvh_build(const mlbvh_triangle* dTriangles, uint32_t nTriangles, uint32_t buildOption,

@@ -468,7 +468,12 @@ mlbvh_status launch_small_sort(const float* tris, uint32_t n, uint32_t option, u
 
 }  // namespace
 
-size_t build_scratch_bytes(uint32_t n) { return build_layout(n).total; }
+// Just above kFewMax the larger sort tiles need less: the size does not fall
+// there, so that scratch for n triangles serves every smaller build.
+size_t build_scratch_bytes(uint32_t n)
+{
+    return std::max(build_layout(n).total, build_layout(std::min(n, kFewMax)).total);
+}
 
 mlbvh_status sort_leaves(const mlbvh_triangle* dTris, uint32_t n, uint32_t option, mlbvh_aabb* dScene,
                          uint32_t* dKeysOut, uint32_t* dIdxOut, void* dScratch, cudaStream_t stream,
@@ -550,7 +555,7 @@ mlbvh_status build(const mlbvh_triangle* dTris, uint32_t n, uint32_t option, mlb
     if (!aligned16(dTris) || !aligned16(dNodes) || !aligned16(dScratch) || !aligned16(dRoot) || !aligned16(dScene) ||
         !aligned16(dKeysOut) || !aligned16(dIdxOut) || !aligned16(dDeltasOut))
         return fail(MLBVH_ERR_INVALID_ARG, "device pointers must be 16-byte aligned");
-    if (scratchBytes < build_layout(n).total)
+    if (scratchBytes < build_scratch_bytes(n))
         return fail(MLBVH_ERR_INVALID_ARG, "scratch smaller than mlbvh_build_scratch_bytes(n)");
     SortedLeaves sl;
     mlbvh_status st = sort_leaves(dTris, n, option, dScene, dKeysOut, dIdxOut, dScratch, stream, spinLimit, &sl);
