@@ -123,13 +123,14 @@ __device__ __forceinline__ float unordered(uint32_t k)
 }
 
 // Mesh of sorted position / tile / ray x: the largest m with off[m] <= x,
-// for off[0] <= x < off[count].
-__device__ __forceinline__ uint32_t find_segment(const uint32_t* __restrict__ off, uint32_t count, uint32_t x)
+// for off[0] <= x < off[count]. kChain: off is written in the build's chain.
+template <bool kChain = false>
+__device__ __forceinline__ uint32_t find_segment(const uint32_t* off, uint32_t count, uint32_t x)
 {
     uint32_t lo = 0, hi = count;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(off + mid) <= x)
+        if ((kChain ? chain_load(off + mid) : __ldg(off + mid)) <= x)
             lo = mid;
         else
             hi = mid;
@@ -242,14 +243,14 @@ __device__ __forceinline__ void stage_floats(float* s, const float* __restrict__
 struct TileWork {
     uint32_t mesh, start, len, first, count;
 };
-__device__ __forceinline__ bool tile_work(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tileStart,
+__device__ __forceinline__ bool tile_work(const uint32_t* __restrict__ off, const uint32_t* tileStart,
                                           uint32_t nMeshes, uint32_t tile, TileWork& w)
 {
-    if (tile >= __ldg(tileStart + nMeshes)) return false;
-    w.mesh = find_segment(tileStart, nMeshes, tile);
+    if (tile >= chain_load(tileStart + nMeshes)) return false;
+    w.mesh = find_segment<true>(tileStart, nMeshes, tile);
     w.start = __ldg(off + w.mesh);
     w.len = __ldg(off + w.mesh + 1) - w.start;
-    w.first = (tile - __ldg(tileStart + w.mesh)) * (uint32_t)sort::kTile;
+    w.first = (tile - chain_load(tileStart + w.mesh)) * (uint32_t)sort::kTile;
     w.count = min((uint32_t)sort::kTile, w.len - w.first);
     return true;
 }
@@ -258,7 +259,7 @@ __device__ __forceinline__ bool tile_work(const uint32_t* __restrict__ off, cons
 // Every CTA also zeroes its share of [zeroBegin, zeroBegin + zeroWords).
 __global__ void __launch_bounds__(kTileThreads)
     k_batch_bounds(const float* __restrict__ tris, uint32_t n, const uint32_t* __restrict__ off, uint32_t nMeshes,
-                   const uint32_t* __restrict__ tileStart, uint32_t* __restrict__ bounds,
+                   const uint32_t* tileStart, uint32_t* __restrict__ bounds,
                    uint32_t* __restrict__ zeroBegin, size_t zeroWords)
 {
     chain_begin();
@@ -318,7 +319,7 @@ __global__ void __launch_bounds__(kTileThreads)
 template <int kBits>
 __global__ void __launch_bounds__(kTileThreads)
     k_batch_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const uint32_t* __restrict__ off,
-                 uint32_t nMeshes, const uint32_t* __restrict__ tileStart, const uint32_t* __restrict__ bounds,
+                 uint32_t nMeshes, const uint32_t* tileStart, const uint32_t* bounds,
                  uint32_t* __restrict__ keys, uint32_t* __restrict__ histogram, uint32_t* __restrict__ handoff,
                  mlbvh_aabb* __restrict__ meshAABBs, uint32_t* __restrict__ treeFlags)
 {
@@ -333,9 +334,9 @@ __global__ void __launch_bounds__(kTileThreads)
     for (int i = threadIdx.x; i < kPasses * kBins; i += kTileThreads) s_hist[i] = 0u;
     const uint32_t* mb = bounds + 6 * (size_t)w.mesh;
     if (w.first == 0 && meshAABBs && threadIdx.x < 6)
-        reinterpret_cast<float*>(meshAABBs + w.mesh)[threadIdx.x] = unordered(__ldcg(mb + threadIdx.x));
-    const f3 lower = mk(unordered(__ldcg(mb)), unordered(__ldcg(mb + 1)), unordered(__ldcg(mb + 2)));
-    const f3 upper = mk(unordered(__ldcg(mb + 3)), unordered(__ldcg(mb + 4)), unordered(__ldcg(mb + 5)));
+        reinterpret_cast<float*>(meshAABBs + w.mesh)[threadIdx.x] = unordered(chain_load(mb + threadIdx.x));
+    const f3 lower = mk(unordered(chain_load(mb)), unordered(chain_load(mb + 1)), unordered(chain_load(mb + 2)));
+    const f3 upper = mk(unordered(chain_load(mb + 3)), unordered(chain_load(mb + 4)), unordered(chain_load(mb + 5)));
     // hand-off words of the mesh's internal nodes [first, first + count) ∩ [0, len - 1)
     uint32_t* ho = handoff + (w.start - w.mesh);
     for (uint32_t j = w.first + threadIdx.x; j < w.first + w.count && j + 1 < w.len; j += kTileThreads)

@@ -181,7 +181,7 @@ __device__ __forceinline__ uint32_t triangle_key(const float* t, uint32_t option
 // first: the bounds pass has just read the array forwards, so its end is what
 // the L2 still holds.
 __global__ void __launch_bounds__(kKeysThreads)
-    k_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const float* __restrict__ partials,
+    k_keys(const float* __restrict__ tris, uint32_t n, uint32_t option, const float* partials,
            int nPartials, uint32_t* __restrict__ keys, uint32_t* __restrict__ histogram,
            uint32_t* __restrict__ handoff, mlbvh_aabb* __restrict__ sceneOut, uint32_t* __restrict__ treeFlags)
 {
@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(kKeysThreads)
     if (warp == 0) {
         float lo[3] = {kFltMax, kFltMax, kFltMax}, hi[3] = {-kFltMax, -kFltMax, -kFltMax};
         for (int p = lane; p < nPartials; p += 32) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(partials + p * 8));
-            const float4 b = __ldg(reinterpret_cast<const float4*>(partials + p * 8) + 1);
+            const float4 a = chain_load(reinterpret_cast<const float4*>(partials + p * 8));
+            const float4 b = chain_load(reinterpret_cast<const float4*>(partials + p * 8) + 1);
             const float l[3] = {a.x, a.y, a.z}, h[3] = {a.w, b.x, b.y};
 #pragma unroll
             for (int x = 0; x < 3; ++x) {

@@ -6,6 +6,7 @@
 
 #include "../../include/mlbvh.h"
 #include "../../include/mlbvh_device.cuh"
+#include "chain.cuh"
 
 namespace mlbvh {
 
@@ -16,9 +17,9 @@ __device__ __forceinline__ uint32_t exch_acq_rel(uint32_t* p, uint32_t v)
     return old;
 }
 
-__device__ __forceinline__ uint32_t delta_at(const uint32_t* __restrict__ keys, uint32_t i)
+__device__ __forceinline__ uint32_t delta_at(const uint32_t* keys, uint32_t i)
 {
-    return split_delta(keys[i], keys[i + 1]);
+    return split_delta(chain_load(keys + i), chain_load(keys + i + 1));
 }
 
 // A triangle's three corners with three 16-byte loads: the 48-byte window
@@ -78,7 +79,7 @@ __device__ __forceinline__ void leaf_box(const float* __restrict__ tris, uint32_
 // at the range's ends only the one at the end that moved is recomputed. The
 // node array must be 16-byte aligned.
 __device__ __forceinline__ void climb(uint32_t n, uint32_t i, uint32_t tri, f3 lo, f3 hi,
-                                      const uint32_t* __restrict__ sortedKeys,
+                                      const uint32_t* sortedKeys,
                                       mlbvh_internal_node* __restrict__ nodes, uint32_t* __restrict__ handoff,
                                       mlbvh_node_index* __restrict__ root)
 {

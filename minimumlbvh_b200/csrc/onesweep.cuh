@@ -84,18 +84,18 @@ struct MeshSegments {
     uint32_t stride;
     __device__ __forceinline__ bool resolve(uint32_t tile, Segment& s) const
     {
-        if (tile >= __ldcg(tileStart + nSegments)) return false;
+        if (tile >= chain_load(tileStart + nSegments)) return false;
         uint32_t lo = 0, hi = nSegments;  // tileStart[lo] <= tile < tileStart[hi]
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldcg(tileStart + mid) <= tile)
+            if (chain_load(tileStart + mid) <= tile)
                 lo = mid;
             else
                 hi = mid;
         }
-        s.start = __ldcg(offsets + lo);
-        s.len = __ldcg(offsets + lo + 1) - s.start;
-        s.firstTile = __ldcg(tileStart + lo);
+        s.start = __ldg(offsets + lo);
+        s.len = __ldg(offsets + lo + 1) - s.start;
+        s.firstTile = chain_load(tileStart + lo);
         s.counts = counts + (size_t)lo * stride;
         return true;
     }
@@ -148,8 +148,8 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp /*kW
 // array that leaves multiprocessors idle is cut into smaller tiles.
 template <int kBits, bool kFirst, class Segments, int kPer = kItems>
 __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
-    k_onesweep(const uint32_t* __restrict__ keysIn, uint32_t* __restrict__ keysOut,
-               const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ valsOut, int shift, Segments segs,
+    k_onesweep(const uint32_t* keysIn, uint32_t* __restrict__ keysOut,
+               const uint32_t* valsIn, uint32_t* __restrict__ valsOut, int shift, Segments segs,
                uint32_t* __restrict__ lookback, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ errorWord,
                uint32_t spinLimit)
 {
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
 #pragma unroll
         for (int j = 0; j < kDPT; ++j) {
             uint32_t total;
-            const uint32_t excl = block_scan(__ldg(seg.counts + j * kThreads + tid), s_scan, &total);
+            const uint32_t excl = block_scan(chain_load(seg.counts + j * kThreads + tid), s_scan, &total);
             digitBase[j] = running + excl;
             running += total;
         }
@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
     for (int k = 0; k < kPer; ++k) {
         const uint32_t li = localBase + k * 32 + lane;
         const bool valid = li < seg.len;
-        key[k] = valid ? __ldg(keysIn + seg.start + li) : 0xFFFFFFFFu;
-        val[k] = kFirst ? li : (valid ? __ldg(valsIn + seg.start + li) : 0u);
+        key[k] = valid ? chain_load(keysIn + seg.start + li) : 0xFFFFFFFFu;
+        val[k] = kFirst ? li : (valid ? chain_load(valsIn + seg.start + li) : 0u);
     }
     const uint32_t lanesBelow = (1u << lane) - 1u;
     uint32_t* myHist = s_warpHist + warp * kBins;

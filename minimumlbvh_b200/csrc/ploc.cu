@@ -633,7 +633,7 @@ __device__ void place_all(const PlocArgs& a)
 }
 
 __global__ void __launch_bounds__(kInitThreads)
-    k_ploc_init(const float* __restrict__ tris, const uint32_t* __restrict__ sortedIdx, uint32_t n,
+    k_ploc_init(const float* __restrict__ tris, const uint32_t* sortedIdx, uint32_t n,
                 float4* __restrict__ clusters, unsigned long long* __restrict__ flags, uint32_t nFlags,
                 PlocControl* __restrict__ ctl, unsigned long long* __restrict__ info)
 {
@@ -648,7 +648,7 @@ __global__ void __launch_bounds__(kInitThreads)
         ctl->placeNext = 0;
     }
     for (uint32_t i = g; i < n; i += stride) {
-        uint32_t tri = sortedIdx[i];
+        uint32_t tri = chain_load(sortedIdx + i);
         if (tri >= n) tri = 0;  // only after a sort whose bounded wait gave up (error word set)
         f3 lo, hi;
         leaf_box(tris, n, tri, lo, hi);

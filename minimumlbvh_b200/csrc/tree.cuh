@@ -215,7 +215,7 @@ __device__ __forceinline__ Box shuffle_down(const Box& b, int o)
 }
 __device__ __forceinline__ Box load_box(const float4* b, uint32_t i)
 {
-    const float4 lo = __ldcg(b + 2 * (size_t)i), hi = __ldcg(b + 2 * (size_t)i + 1);
+    const float4 lo = chain_load(b + 2 * (size_t)i), hi = chain_load(b + 2 * (size_t)i + 1);
     return Box{mk(lo.x, lo.y, lo.z), mk(hi.x, hi.y, hi.z)};
 }
 __device__ __forceinline__ void store_box(float4* b, uint32_t i, const Box& v)
@@ -233,7 +233,7 @@ __device__ __forceinline__ void reduce_block(const Level& from, const Level& to,
     uint32_t m = 0;
     if (has) {
         b = load_box(from.box, 32 * block + lane);
-        m = __ldcg(from.max + 32 * (size_t)block + lane);
+        m = chain_load(from.max + 32 * (size_t)block + lane);
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -257,7 +257,7 @@ static __global__ void __launch_bounds__(128) k_tree_groups(Scratch sc)
 {
     chain_begin();
     const uint32_t groups = (sc.nTiles + 31) / 32, g = (blockIdx.x * 128 + threadIdx.x) >> 5;
-    if (g >= groups || (__ldcg(sc.flags) & (kNaN | kSkip))) return;
+    if (g >= groups || (chain_load(sc.flags) & (kNaN | kSkip))) return;
     reduce_block(sc.level[0], sc.level[1], sc.nTiles, g);
     if (groups <= 32) return;
     uint32_t last = 0;
@@ -282,8 +282,8 @@ __device__ __forceinline__ void copy16(void* dst, const void* src)
 
 template <class Trees>
 __global__ void __launch_bounds__(kTile, kTileCtas)
-    k_tree_tiles(const float* __restrict__ tris, Trees trees, const uint32_t* __restrict__ keys,
-                 const uint32_t* __restrict__ idx, mlbvh_internal_node* __restrict__ nodes,
+    k_tree_tiles(const float* __restrict__ tris, Trees trees, const uint32_t* keys,
+                 const uint32_t* idx, mlbvh_internal_node* __restrict__ nodes,
                  mlbvh_node_index* __restrict__ roots, uint8_t* __restrict__ deltasOut, Scratch sc)
 {
     // the joins of 2^k leaves from each leaf on (to the end of its warp), then the assembled nodes by word
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kTile, kTileCtas)
     __shared__ Box s_warpBox[kWarps], s_before[kWarps], s_after[kWarps];
     __shared__ uint32_t s_mesh[Trees::kMany ? kTile : 1];
     chain_begin();
-    if (__ldcg(sc.flags) & (kNaN | kSkip)) return;  // the whole CTA: set before this launch
+    if (chain_load(sc.flags) & (kNaN | kSkip)) return;  // the whole CTA: set before this launch
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = sc.n;
     float4* const window = s_tri + 3 * tid;
@@ -312,9 +312,9 @@ __global__ void __launch_bounds__(kTile, kTileCtas)
     auto first_word = [&](const Segment& s, uint32_t tri) { return 9 * ((size_t)s.start + tri); };
     auto load_ahead = [&](uint32_t g, Ahead& a) {
         if (g < n) {
-            a.tri = __ldg(idx + g);
-            a.key0 = __ldg(keys + g);
-            a.key1 = g + 1 < n ? __ldg(keys + g + 1) : 0u;
+            a.tri = chain_load(idx + g);
+            a.key0 = chain_load(keys + g);
+            a.key1 = g + 1 < n ? chain_load(keys + g + 1) : 0u;
         }
     };
     auto copy_window = [&](uint32_t g, const Segment& s, Ahead& a) {
@@ -682,7 +682,7 @@ struct Sum {
 // Joins entries [from, to] of one block of a level (8 per lane, those outside
 // replaced by the nearest inside: joining an entry twice changes nothing) onto
 // acc's outer end. Every lane of the side gets the result.
-__device__ __forceinline__ void join_entries(Sum& acc, const float4* __restrict__ boxes, uint32_t from, uint32_t to,
+__device__ __forceinline__ void join_entries(Sum& acc, const float4* boxes, uint32_t from, uint32_t to,
                                              const Side& sd)
 {
     const uint32_t base = (from & ~31u) + 8 * sd.r;
@@ -714,7 +714,7 @@ __device__ __forceinline__ uint32_t find_tile(const Scratch& sc, uint32_t i, uin
         allowed &= 0xFFFFFFFFu >> (32u - min(32u, entries(l) - base));
         if (allowed == 0u) return kNone;
         const Level level = level_of(sc, l);
-        const uint2 w = __ldg(reinterpret_cast<const uint2*>(level.max + base) + sd.r);
+        const uint2 w = chain_load(reinterpret_cast<const uint2*>(level.max + base) + sd.r);
         uint32_t m = (bytes_ge(w.x, d) | bytes_ge(w.y, d) << 4) << (8 * sd.r);
         m |= __shfl_xor_sync(sd.lanes, m, 1);
         m |= __shfl_xor_sync(sd.lanes, m, 2);
@@ -754,20 +754,20 @@ __device__ __forceinline__ uint32_t find_tile(const Scratch& sc, uint32_t i, uin
 
 template <class Trees>
 __global__ void __launch_bounds__(kCrossThreads)
-    k_tree_cross(const float* __restrict__ tris, Trees trees, const uint32_t* __restrict__ keys,
-                 const uint32_t* __restrict__ idx, mlbvh_internal_node* __restrict__ nodes,
+    k_tree_cross(const float* __restrict__ tris, Trees trees, const uint32_t* keys,
+                 const uint32_t* idx, mlbvh_internal_node* __restrict__ nodes,
                  mlbvh_node_index* __restrict__ roots, uint8_t* __restrict__ deltasOut, uint32_t* __restrict__ handoff,
                  Scratch sc)
 {
     __shared__ uint32_t s_far[kCrossNodes], s_nFar;
     chain_begin();
     const uint32_t thread = blockIdx.x * kCrossThreads + threadIdx.x, threads = gridDim.x * kCrossThreads;
-    const uint32_t flags = __ldcg(sc.flags);
+    const uint32_t flags = chain_load(sc.flags);
     if (flags & kSkip) return;
     if (flags) {  // NaN or too many records: every leaf climbs
         for (uint32_t g = thread; g < sc.n; g += threads) {
             const Segment seg = trees.of(g);
-            const uint32_t tri = idx[g], len = seg.end - seg.start;
+            const uint32_t tri = chain_load(idx + g), len = seg.end - seg.start;
             // k_tree_tiles leaves before its deltas where a centroid is NaN
             if (deltasOut && g + 1 < seg.end) deltasOut[g] = (uint8_t)delta_at(keys, g);
             if (tri >= len) continue;  // a bounded wait of the sort gave up (error word set)
@@ -778,13 +778,13 @@ __global__ void __launch_bounds__(kCrossThreads)
         }
         return;
     }
-    const uint32_t count = min(__ldcg(sc.nRecords), sc.capacity);
+    const uint32_t count = min(chain_load(sc.nRecords), sc.capacity);
     struct Half {  // a record's half, or a tile's box
         Box b;
         uint32_t x, y;
     };
     auto load_half = [&](const float4* r) {
-        const float4 a = __ldg(r), b = __ldg(r + 1);
+        const float4 a = chain_load(r), b = chain_load(r + 1);
         return Half{Box{mk(a.x, a.y, a.z), mk(b.x, b.y, b.z)}, __float_as_uint(a.w), __float_as_uint(b.w)};
     };
     auto tile_box = [&](uint32_t t) { return (const float4*)(sc.level[0].box + 2 * (size_t)t); };
@@ -845,9 +845,9 @@ __global__ void __launch_bounds__(kCrossThreads)
             const uint32_t p = pre.x, d = pre.y & 0xFFu, mesh = pre.y >> 8, l = suf.x, u = suf.y, tile = p / kTile;
             if (d < kInf) {  // else a tree's last leaf, no node
                 const uint32_t tl = max(tile, 1u) - 1, tr = min(tile + 1, sc.nTiles - 1);
-                const uint32_t maxL = __ldg(sc.level[0].max + tl), maxR = __ldg(sc.level[0].max + tr);
-                const uint32_t recL = __ldg(&sc.ends[tl].record0), recR = __ldg(&sc.ends[tr].record0);
-                const uint32_t rankL = __ldg(sc.ends[tl].last + d), rankR = __ldg(sc.ends[tr].first + d);
+                const uint32_t maxL = chain_load(sc.level[0].max + tl), maxR = chain_load(sc.level[0].max + tr);
+                const uint32_t recL = chain_load(&sc.ends[tl].record0), recR = chain_load(&sc.ends[tr].record0);
+                const uint32_t rankL = chain_load(sc.ends[tl].last + d), rankR = chain_load(sc.ends[tr].first + d);
                 Sum acc{own_part(slot, tile, l, u), true};
                 const bool nearL = !(l & kOut) || tile == 0 || maxL >= d, nearR = !(u & kOut) || maxR > d;
                 if (nearL && nearR) {
@@ -877,8 +877,8 @@ __global__ void __launch_bounds__(kCrossThreads)
                 const uint32_t t = find_tile(sc, tile, sd.left ? d : d + 1, acc, sd);
                 e = End{sd.left ? 0u : sc.n - 1, kInf};
                 if (t != kNone)
-                    e = end_in(t, sd.left, __ldg(&sc.ends[t].record0),
-                               sd.left ? __ldg(sc.ends[t].last + d) : __ldg(sc.ends[t].first + d), acc);
+                    e = end_in(t, sd.left, chain_load(&sc.ends[t].record0),
+                               sd.left ? chain_load(sc.ends[t].last + d) : chain_load(sc.ends[t].first + d), acc);
             }
             const Box other = shuffle_xor(acc.b, 4, both);
             const bool otherHas = __shfl_xor_sync(both, acc.has ? 1 : 0, 4) != 0;
