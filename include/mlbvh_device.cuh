@@ -487,6 +487,17 @@ __device__ __forceinline__ bool stackfree_replay_step_lo(uint32_t& curr, uint32_
     }
 }
 
+// What a round of up to kNodes node visits and one leaf test counts towards the
+// limit on a lane's steps: the fewest it can have held, so that no walk ends
+// earlier than step by step (counting every step on its own cost 1 to 4 %).
+// tested: the lane made the round's last step, at a leaf or by the stack-free
+// rules; a lane that did not was at inner nodes throughout.
+template <int kNodes>
+__device__ __forceinline__ constexpr uint32_t phase_steps(bool tested)
+{
+    return tested ? 1u : (uint32_t)kNodes;
+}
+
 // A whole walk of a thread's ray in phases: up to kNodes node visits, then one
 // leaf test. A warp's lanes are at nodes far more often than at leaves, but
 // with one step of either kind at a time nearly every step of the warp has
@@ -498,12 +509,14 @@ template <int kNodes, class Step>
 __device__ __forceinline__ void walk_phases(const uint32_t& curr, const int& depth, Step step)
 {
     bool done = false;
-    for (uint32_t steps = 0; steps < kMaxTraversalSteps; steps += kNodes + 1) {
+    for (uint32_t steps = 0; steps < kMaxTraversalSteps;) {
 #pragma unroll
         for (int k = 0; k < kNodes; ++k)
             if (!done && !(curr & kLeafBit) && depth >= 0) done = step();
-        if (!done && ((curr & kLeafBit) || depth < 0)) done = step();
+        const bool test = !done && ((curr & kLeafBit) || depth < 0);
+        if (test) done = step();
         if (done) return;
+        steps += phase_steps<kNodes>(test);
     }
 }
 

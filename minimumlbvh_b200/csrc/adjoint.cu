@@ -243,12 +243,13 @@ __device__ __forceinline__ void trace_pixels(const DiffScene& sc, float* __restr
                 if (!replay_node<false, kDiffStack>(curr, prev, depth, stack, kDiffThreads, hit.t, sc.nodes, ro, inv,
                                                     0.0f))
                     walking = !replay_pop<false>(curr, depth, stack, kDiffThreads, hit.t);
-        if (walking && ((curr & kLeafBit) || depth < 0)) {
+        const bool test = walking && ((curr & kLeafBit) || depth < 0);
+        if (test) {
             uint32_t nv = 0, nt = 0;
             walking = !stackfree_replay_step<false, false, kDiffStack>(curr, prev, depth, stack, kDiffThreads, hit,
                                                                        sc.nodes, sc.tris, ro, rd, inv, 0.0f, nv, nt);
         }
-        steps += kDiffSteps + 1;
+        steps += phase_steps<kDiffSteps>(test);
         if (steps >= kMaxTraversalSteps) walking = false;
     }
 }

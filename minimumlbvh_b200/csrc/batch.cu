@@ -494,8 +494,9 @@ __global__ void __launch_bounds__(512, 2)
 #pragma unroll
             for (int k = 0; k < kBatchNodeSteps; ++k)
                 if (!done && !(curr & kLeafBit) && depth >= 0) done = step();
-            if (!done && ((curr & kLeafBit) || depth < 0)) done = step();
-            steps += kBatchNodeSteps + 1;
+            const bool test = !done && ((curr & kLeafBit) || depth < 0);
+            if (test) done = step();
+            steps += phase_steps<kBatchNodeSteps>(test);
             if (done || steps >= kMaxTraversalSteps) {
                 hits[2 * (size_t)ray] = make_float4(hit.t, 0.0f, hit.u, hit.v);
                 hits[2 * (size_t)ray + 1] = make_float4(hit.ng.x, hit.ng.y, hit.ng.z, __uint_as_float(hit.tri));

@@ -92,12 +92,13 @@ __device__ __forceinline__ void trace_pool(const float4* __restrict__ rays, floa
             for (int k = 0; k < kNodes; ++k)
                 if (live && !done && !apart() && !(curr & kLeafBit)) done = step();
         }
-        if (live && !done && !apart() && (curr & kLeafBit)) done = step();
+        const bool test = live && !done && !apart() && (curr & kLeafBit);
+        if (test) done = step();
         if (live && !done && apart()) {  // as many steps of either kind
 #pragma unroll 1
             for (int k = 0; k <= kNodes && !done; ++k) done = step();
         }
-        steps += rounds * kNodes + 1;
+        steps += phase_steps<kNodes>(test);
         if (live && (done || steps >= kMaxTraversalSteps)) {
             hits[2 * (size_t)ray] = make_float4(hit.t, 0.0f, hit.u, hit.v);
             hits[2 * (size_t)ray + 1] = make_float4(hit.ng.x, hit.ng.y, hit.ng.z, __uint_as_float(hit.tri));

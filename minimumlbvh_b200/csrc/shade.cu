@@ -622,13 +622,14 @@ __global__ void __launch_bounds__(kAoThreads, MinBlocksOf<Tree>::value)
                     occluded = hit.t != radius;
                 }
             }
-        if (live && ((curr & kLeafBit) || depth < 0)) {
+        const bool test = live && ((curr & kLeafBit) || depth < 0);
+        if (test) {
             if (tree.template step<true, kCount>(ctx, curr, prev, depth, stack, hit, origin, dir, inv, cnt, fits)) {
                 live = false;
                 occluded = hit.t != radius;
             }
         }
-        steps += StepsOf<Tree>::value + 1;
+        steps += phase_steps<StepsOf<Tree>::value>(test);
         if (steps >= kMaxTraversalSteps) live = false;
         // one atomic per pixel among the lanes whose ray just ended occluded
         uint32_t pending = __ballot_sync(0xffffffffu, occluded);
@@ -870,8 +871,9 @@ __global__ void __launch_bounds__(kPtThreads, kPtWarps * 32 / kPtThreads)
 #pragma unroll
         for (int k = 0; k < kPtSteps; ++k)
             if (walking && !done && !(curr & kLeafBit) && depth >= 0) done = step();
-        if (walking && !done && ((curr & kLeafBit) || depth < 0)) done = step();
-        steps += kPtSteps + 1;
+        const bool test = walking && !done && ((curr & kLeafBit) || depth < 0);
+        if (test) done = step();
+        steps += phase_steps<kPtSteps>(test);
         if (done || steps >= kMaxTraversalSteps) walking = false;
     }
 }
