@@ -55,7 +55,7 @@ constexpr uint32_t kErrOffsets = 2u;
 // header words
 constexpr int kHdrError = 0;
 constexpr int kHdrTickets = 1;  // 4 tile tickets, one per sort pass
-constexpr int kHdrTreeFlags = 5;  // tree::Scratch::flags; the record count follows
+constexpr int kHdrTreeFlags = 5;  // tree::Scratch::flags; the record count and the next tile follow
 constexpr int kHdrQueue = 8;    // traversal queue counter
 
 struct BatchLayout {

@@ -44,7 +44,7 @@ constexpr int kKeysThreads = 256;
 // 450,000: 136, 126, 129).
 constexpr uint32_t kFewMax = 3 * 148 * sort::kThreads * sort::kFewItems;
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
-constexpr int kHdrTreeFlags = 5;  // header word of tree::Scratch::flags; the record count follows
+constexpr int kHdrTreeFlags = 5;  // header word of tree::Scratch::flags; the record count and the next tile follow
 
 // Arrays up to this size take one CTA from the triangles to the sorted keys
 // (k_small_sort) instead of the bounds, key and sort kernels, whose launches and
@@ -57,7 +57,7 @@ constexpr uint32_t kSmallMax = 4 * kSmallThreads;
 // Scratch layout of one build (offsets from the caller's dScratch). The
 // leading region [header, partials) is zeroed by k_scene_bounds on every build.
 struct BuildLayout {
-    size_t header;     // u32 error word, u32 tile counters[4], u32 tree flags, u32 tree records
+    size_t header;     // u32 error word, u32 tile counters[4], u32 tree flags, tree records, next tile
     size_t histogram;  // 4 x 256 u32
     size_t lookback;   // 4 x tiles x 256 u32
     size_t treeCounts; // tree::count_bytes(n)

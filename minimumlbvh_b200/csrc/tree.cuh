@@ -33,8 +33,11 @@
 //
 // The join is associative only without NaN (right < left is false for either
 // order of a NaN). k_keys marks builds with a NaN centroid, and a build whose
-// records do not fit (runs of equal keys across tiles) is marked too: those
-// trees are climbed leaf by leaf (climb.cuh) by k_tree_cross instead.
+// records do not fit (runs of equal keys across tiles, meshes of a few triangles)
+// is marked too: those trees are climbed leaf by leaf (climb.cuh), by
+// k_tree_groups, or by k_tree_cross in builds that have no groups. Whole builds
+// with one NaN (without): 1,000 triangles 43 us (23), 213k 113 (79), 4M 683
+// (518); 213k in runs of 300 equal keys 499, 1,000 meshes of 1-16 triangles 134.
 //
 // Measured (B200, kernel times): 4M-triangle soup 225 + 5 + 34 us against 401
 // us for the climb with shared-memory hand-offs per tile; 213k-triangle
@@ -70,6 +73,8 @@ constexpr uint32_t kSkip = 4u;             // flag bit: build nothing (bad batch
 constexpr int kTileCtas = 3;
 constexpr int kCrossThreads = 128;
 constexpr uint32_t kCrossNodes = 64;  // records per CTA and round of k_tree_cross
+constexpr uint32_t kGroupThreads = 64;
+constexpr int kGroupCtas = 32;  // resident CTAs per SM of k_tree_groups: 2,048 threads
 constexpr uint32_t kCrossLanes = 8;  // lanes per crossing node
 
 struct Box {
@@ -110,6 +115,7 @@ struct Ends {
 struct Scratch {
     uint32_t* flags;      // kNaN | kFull | kSkip; zeroed before the keys are made
     uint32_t* nRecords;   // zeroed with flags
+    uint32_t* nextTile;   // of the climb; zeroed with flags
     Ends* ends;           // per tile
     Record* records;
     uint32_t capacity;    // records
@@ -145,6 +151,7 @@ inline Scratch place(uint32_t n, char* summary, uint32_t* counts, uint32_t* flag
     Scratch s;
     s.flags = flags;
     s.nRecords = flags + 1;
+    s.nextTile = flags + 2;
     s.n = n;
     s.nTiles = tiles_of(n);
     s.counts = counts;
@@ -252,12 +259,65 @@ __device__ __forceinline__ void reduce_block(const Level& from, const Level& to,
     }
 }
 
-// One warp per group; the last group of a super to finish reduces it.
-static __global__ void __launch_bounds__(128) k_tree_groups(Scratch sc)
+// The build as a climb (climb.cuh): a thread per leaf, CTAs of kLeaves threads
+// that take the tiles in order, each when its last one is done. (A CTA that
+// falls behind with tiles of its own is the second to arrive everywhere and
+// climbs ever more: 4M triangles with a NaN took 1,072 us with the tiles dealt
+// out in turn and take 683 now; 1M in runs of 1,000 equal keys 2,886 us with the
+// next tile taken before the last one's climbs end, 1,646 now.)
+inline __host__ __device__ bool grouped(const Scratch& sc) { return sc.nTiles > 32; }
+template <uint32_t kLeaves, class Trees>
+__device__ __forceinline__ void climb_tiles(const float* __restrict__ tris, const Trees& trees, const uint32_t* keys,
+                                            const uint32_t* idx, mlbvh_internal_node* __restrict__ nodes,
+                                            mlbvh_node_index* __restrict__ roots, uint8_t* __restrict__ deltasOut,
+                                            uint32_t* __restrict__ handoff, const Scratch& sc)
+{
+    __shared__ TileClimbShared<kLeaves> s_climb;
+    __shared__ uint32_t s_t0;
+    for (;;) {
+        __syncthreads();  // no tile is taken before the last one is done
+        if (threadIdx.x == 0) s_t0 = atomicAdd(sc.nextTile, 1u) * kLeaves;
+        __syncthreads();
+        const uint32_t t0 = s_t0;
+        if (t0 >= sc.n) return;
+        const uint32_t g = t0 + threadIdx.x;
+        Segment seg{sc.n, sc.n, 0u};
+        uint32_t tri = 0xFFFFFFFFu;
+        f3 lo = mk(0.0f, 0.0f, 0.0f), hi = lo;
+        if (g < sc.n) {
+            seg = trees.of(g);
+            tri = chain_load(idx + g);
+            // k_tree_tiles leaves before its deltas where a centroid is NaN
+            if (deltasOut && g + 1 < seg.end) deltasOut[g] = (uint8_t)delta_at(keys, g);
+            // tri >= the tree's size only after a sort whose bounded wait gave up (error word set)
+            if (tri < seg.end - seg.start)
+                leaf_box(tris + 9 * (size_t)seg.start, seg.end - seg.start, tri, lo, hi);
+        }
+        tile_climb_prepare(s_climb, keys, sc.n, t0, seg.start, seg.end);
+        if (tri < seg.end - seg.start)
+            climb_tile(s_climb, t0 - seg.start, seg.end - seg.start, g - seg.start, tri, lo, hi, keys + seg.start,
+                       nodes + (seg.start - seg.mesh), handoff + (seg.start - seg.mesh), roots + seg.mesh);
+    }
+}
+
+// One warp per group; the last group of a super to finish reduces it. Builds
+// that cannot take the range queries are climbed here: with 32 registers twice
+// as many leaves are under way as k_tree_cross would hold, and the climb is a
+// chain of hand-offs.
+template <class Trees>
+__global__ void __launch_bounds__(kGroupThreads, kGroupCtas)
+    k_tree_groups(const float* __restrict__ tris, Trees trees, const uint32_t* keys, const uint32_t* idx,
+                  mlbvh_internal_node* __restrict__ nodes, mlbvh_node_index* __restrict__ roots,
+                  uint8_t* __restrict__ deltasOut, uint32_t* __restrict__ handoff, Scratch sc)
 {
     chain_begin();
-    const uint32_t groups = (sc.nTiles + 31) / 32, g = (blockIdx.x * 128 + threadIdx.x) >> 5;
-    if (g >= groups || (chain_load(sc.flags) & (kNaN | kSkip))) return;
+    const uint32_t flags = chain_load(sc.flags);
+    if (flags) {
+        if (!(flags & kSkip)) climb_tiles<kGroupThreads>(tris, trees, keys, idx, nodes, roots, deltasOut, handoff, sc);
+        return;
+    }
+    const uint32_t groups = (sc.nTiles + 31) / 32, g = (blockIdx.x * kGroupThreads + threadIdx.x) >> 5;
+    if (g >= groups) return;
     reduce_block(sc.level[0], sc.level[1], sc.nTiles, g);
     if (groups <= 32) return;
     uint32_t last = 0;
@@ -761,21 +821,10 @@ __global__ void __launch_bounds__(kCrossThreads)
 {
     __shared__ uint32_t s_far[kCrossNodes], s_nFar;
     chain_begin();
-    const uint32_t thread = blockIdx.x * kCrossThreads + threadIdx.x, threads = gridDim.x * kCrossThreads;
     const uint32_t flags = chain_load(sc.flags);
     if (flags & kSkip) return;
     if (flags) {  // NaN or too many records: every leaf climbs
-        for (uint32_t g = thread; g < sc.n; g += threads) {
-            const Segment seg = trees.of(g);
-            const uint32_t tri = chain_load(idx + g), len = seg.end - seg.start;
-            // k_tree_tiles leaves before its deltas where a centroid is NaN
-            if (deltasOut && g + 1 < seg.end) deltasOut[g] = (uint8_t)delta_at(keys, g);
-            if (tri >= len) continue;  // a bounded wait of the sort gave up (error word set)
-            f3 lo, hi;
-            leaf_box(tris + 9 * (size_t)seg.start, len, tri, lo, hi);
-            climb(len, g - seg.start, tri, lo, hi, keys + seg.start, nodes + (seg.start - seg.mesh),
-                  handoff + (seg.start - seg.mesh), roots + seg.mesh);
-        }
+        if (!grouped(sc)) climb_tiles<kCrossThreads>(tris, trees, keys, idx, nodes, roots, deltasOut, handoff, sc);
         return;
     }
     const uint32_t count = min(chain_load(sc.nRecords), sc.capacity);
@@ -902,11 +951,18 @@ inline mlbvh_status launch(const float* tris, const Trees& trees, const uint32_t
     launch_chained(k_tree_tiles<Trees>, tileBlocks, kTile, 0, stream, tris, trees, keys, idx, nodes, roots, deltasOut,
                    sc);
     MLBVH_CHECK_LAUNCH("k_tree_tiles");
-    if (sc.nTiles > 32) {
-        launch_chained(k_tree_groups, (up32(sc.nTiles) + 3) / 4, 128, 0, stream, sc);
+    uint32_t blocks = std::min<uint32_t>(sc.n / 24 / kCrossNodes + 1, 32u * (uint32_t)sms);
+    // a kernel that may have to climb gets a thread per leaf, up to what is resident
+    if (grouped(sc)) {
+        const uint32_t leafBlocks =
+            std::max(std::min<uint32_t>((sc.n + kGroupThreads - 1) / kGroupThreads, kGroupCtas * (uint32_t)sms),
+                     (up32(sc.nTiles) + kGroupThreads / 32 - 1) / (kGroupThreads / 32));
+        launch_chained(k_tree_groups<Trees>, leafBlocks, kGroupThreads, 0, stream, tris, trees, keys, idx, nodes, roots,
+                       deltasOut, handoff, sc);
         MLBVH_CHECK_LAUNCH("k_tree_groups");
+    } else {
+        blocks = std::max<uint32_t>(blocks, (sc.n + kCrossThreads - 1) / kCrossThreads);
     }
-    const uint32_t blocks = std::min<uint32_t>(sc.n / 24 / kCrossNodes + 1, 32u * (uint32_t)sms);
     launch_chained(k_tree_cross<Trees>, blocks, kCrossThreads, 0, stream, tris, trees, keys, idx, nodes, roots,
                    deltasOut, handoff, sc);
     MLBVH_CHECK_LAUNCH("k_tree_cross");
