@@ -20,6 +20,11 @@ namespace {
 
 constexpr int kNodeSteps = 4;  // node visits per leaf test (2: 5 % slower)
 constexpr int kPoolWarps = 32;  // resident warps per SM of the pooled trace kernel (64 registers)
+template <bool kAny>
+constexpr int kEachWarps = kAny ? 36 : 32;  // one ray per thread (56 and 64 registers)
+// rays per SM that run one per thread: to the resident ones; any hit, whose pool spills, to 1.75 times as many
+template <bool kAny>
+constexpr EachRange kEachRange = kAny ? EachRange{0, 2016} : EachRange{96, 1024};
 
 constexpr int kQuantiseThreads = 256;
 __device__ __forceinline__ void leaf_box(const float* __restrict__ tris, uint32_t t, f3& lo, f3& hi)
@@ -205,14 +210,14 @@ __global__ void __launch_bounds__(kQuantiseThreads)
 // memory (quantised_replay_step), which returns the same Hit records.
 // counts (may be null): per ray, internal-node visits, triangle tests and
 // parent loads at counts[i], counts[pool.n + i], counts[2n + i].
-template <bool kAny, int kDepth, bool kCount>
-__global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
+template <bool kAny, int kDepth, bool kCount, bool kEach>
+__global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps<kAny> : kPoolWarps) * 32 / kRayThreads<kEach>)
     k_trace_quantised(const mlbvh_qnode* __restrict__ qnodes, const uint32_t* __restrict__ parents,
                       const mlbvh_qtri* __restrict__ qtris, const mlbvh_qheader* __restrict__ header,
                       const float4* __restrict__ rays, float4* __restrict__ hits,
                       uint32_t* __restrict__ counts, RayPool pool)
 {
-    __shared__ typename ReplayStack<kAny>::Entry s_stack[kDepth > 0 ? kDepth : 1][kPoolThreads];
+    __shared__ typename ReplayStack<kAny>::Entry s_stack[kDepth > 0 ? kDepth : 1][kRayThreads<kEach>];
     const uint32_t root = __ldg(&header->root);
     QParams qp{__ldg(&header->eBase), __ldg(&header->status), false};
     f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
@@ -220,7 +225,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
     HitRecord hit;
     uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0, nu = 0;
     int depth = 0;
-    trace_pool<kNodeSteps>(
+    trace_rays<kEach, kNodeSteps, 1>(
         rays, hits, pool, hit, curr,
         [&](uint32_t, float4 a, float4 b) {
             ro = mk(a.x, a.y, a.z);
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
                                                     nt, nu);
             else
                 return quantised_replay_step<kAny, kCount, kDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                                   kPoolThreads, hit, qnodes, parents, qtris, qp, ro,
+                                                                   kRayThreads<kEach>, hit, qnodes, parents, qtris, qp, ro,
                                                                    rd, inv, tmin, nv, nt, nu);
         },
         [&](uint32_t i) {
@@ -259,10 +264,10 @@ void launch_trace_quantised(cudaStream_t stream, const mlbvh_qnode* q, const uin
                             uint32_t* counts)
 {
     const RayPool pool = ray_pool(n, device_sm_count(), kPoolWarps);
-    if (counts)
-        k_trace_quantised<kAny, kDepth, true><<<pool.ctas, kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, counts, pool);
-    else
-        k_trace_quantised<kAny, kDepth, false><<<pool.ctas, kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, nullptr, pool);
+    const bool each = kEachRange<kAny>.has(n, device_sm_count());
+    const auto kernel = counts ? (each ? k_trace_quantised<kAny, kDepth, true, true> : k_trace_quantised<kAny, kDepth, true, false>)
+                               : (each ? k_trace_quantised<kAny, kDepth, false, true> : k_trace_quantised<kAny, kDepth, false, false>);
+    kernel<<<ray_ctas(pool, each), each ? kEachThreads : kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, counts, pool);
 }
 
 template <bool kAny>

@@ -19,25 +19,32 @@ namespace {
 constexpr int kNodeSteps = 4;  // node visits per leaf test (2-4 within 4 %)
 constexpr int kPoolWarps = 32;  // resident warps per SM of the pooled trace kernel (64 registers)
 
+constexpr int kEachWarps = 36;  // one ray per thread (56 registers)
+// rays per SM that run one per thread: to one and a quarter times the resident ones, any hit; to the resident ones
+template <bool kAny>
+constexpr EachRange kEachRange = kAny ? EachRange{32, 1440} : EachRange{96, 1152};
+
+constexpr int kFewRounds = 3;  // (257 to 4,000 rays: 1M soup 3 to 7 % faster than 1, heightfield 0 to 6 % slower)
+
 constexpr int kTraceThreads = 64;  // of the one-ray-per-thread walks
 
 constexpr int kReplayDepth = 16;  // stack entries per ray of the replay walk
 
 // intersect_stackfree's Hit records through the replay walk.
-template <bool kAny>
-__global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
+template <bool kAny, bool kEach>
+__global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps : kPoolWarps) * 32 / kRayThreads<kEach>)
     k_trace_replay(const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
                    const float* __restrict__ tris, const float4* __restrict__ rays, float4* __restrict__ hits,
                    RayPool pool)
 {
-    __shared__ typename ReplayStack<kAny>::Entry s_stack[kReplayDepth][kPoolThreads];
+    __shared__ typename ReplayStack<kAny>::Entry s_stack[kReplayDepth][kRayThreads<kEach>];
     const uint32_t root = __ldg(rootPtr);
     f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
     float tmin = 0.0f;
     HitRecord hit;
     uint32_t curr = root, prev = kInvalid, nv = 0, nt = 0;
     int depth = 0;
-    trace_pool<kNodeSteps>(
+    trace_rays<kEach, kNodeSteps, kFewRounds>(
         rays, hits, pool, hit, curr,
         [&](uint32_t, float4 a, float4 b) {
             ro = mk(a.x, a.y, a.z);
@@ -52,7 +59,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps * 32 / kPoolThreads)
         [&] { return depth < 0; },
         [&] {
             return stackfree_replay_step<kAny, false, kReplayDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                                    kPoolThreads, hit, nodes, tris, ro, rd, inv, tmin,
+                                                                    kRayThreads<kEach>, hit, nodes, tris, ro, rd, inv, tmin,
                                                                     nv, nt);
         },
         [](uint32_t) {});
@@ -114,10 +121,11 @@ mlbvh_status trace(const mlbvh_internal_node* dNodes, const mlbvh_node_index* dR
     case MLBVH_TRAVERSAL_STACKFREE:  // the replay walk's Hit records are the stack-free walk's
     case MLBVH_TRAVERSAL_REPLAY: {
         const RayPool pool = ray_pool(nRays, device_sm_count(), kPoolWarps);
-        if (any)
-            k_trace_replay<true><<<pool.ctas, kPoolThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, pool);
-        else
-            k_trace_replay<false><<<pool.ctas, kPoolThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits, pool);
+        const bool each = (any ? kEachRange<true> : kEachRange<false>).has(nRays, device_sm_count());
+        const auto kernel = any ? (each ? k_trace_replay<true, true> : k_trace_replay<true, false>)
+                                : (each ? k_trace_replay<false, true> : k_trace_replay<false, false>);
+        kernel<<<ray_ctas(pool, each), each ? kEachThreads : kPoolThreads, 0, stream>>>(dNodes, dRoot, tris, rays, hits,
+                                                                                      pool);
         break;
     }
     case MLBVH_TRAVERSAL_STACKFULL:

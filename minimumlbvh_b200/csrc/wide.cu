@@ -5,6 +5,8 @@
 // binary internal node i, written by one thread with no order between slots:
 // the walk starts at the root's slot and only ever follows child indices,
 // which name the slots of their own expansions.
+#include <type_traits>
+
 #include "capi_internal.h"
 #include "../../include/mlbvh_device.cuh"
 #include "ray_pool.cuh"
@@ -17,6 +19,12 @@ constexpr int kReplayDepth = 16;  // stack entries of the binary replay walk
 // resident warps per SM of the trace kernel, closest hit and any hit
 template <bool kAny>
 constexpr int kPoolWarps = kAny ? 32 : 28;  // (24 / 28 / 32, closest: camera rays 401 / 373 / 413 us, quantised 464 / 437 / 512)
+template <bool kAny>
+constexpr int kEachWarps = kAny ? 36 : 32;  // one ray per thread (56 and 64 registers)
+// rays per SM that run one per thread: to one and a quarter times the resident ones, any hit; to the resident ones
+template <bool kAny>
+constexpr EachRange kEachRange = kAny ? EachRange{32, 1440} : EachRange{96, 1024};
+constexpr int kFewRounds = 3;  // closest hit, FP32 slots; quantised ones 8 to 14 % faster with 1, any hit up to 10 %
 constexpr int kNodeSteps = 3;  // slot visits per leaf test (2 and 4 within 3 %)
 struct WideKid {
     uint32_t name;  // internal index, kLeafBit | leaf position, or kWideEmpty
@@ -185,8 +193,8 @@ __global__ void __launch_bounds__(kWideThreads)
 // sends every ray to the binary tree, and qwide_ray_fits the rays it rejects:
 // to the stack-free walk, or for closest hits without counters to the replay
 // walk, which returns the same Hit records.
-template <bool kAny, bool kCount, bool kQuant, class Slot>
-__global__ void __launch_bounds__(kPoolThreads, kPoolWarps<kAny> * 32 / kPoolThreads)
+template <bool kAny, bool kCount, bool kQuant, bool kEach, class Slot>
+__global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps<kAny> : kPoolWarps<kAny>) * 32 / kRayThreads<kEach>)
     k_trace_wide(const Slot* __restrict__ slots, const uint32_t* __restrict__ status,
                  const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
                  const float* __restrict__ tris, const mlbvh_qtri* __restrict__ leafTris,
@@ -194,7 +202,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps<kAny> * 32 / kPoolThr
                  uint32_t* __restrict__ counts, RayPool pool)
 {
     using Entry = typename ReplayStack<kAny>::Entry;
-    __shared__ Entry s_stack[kWideDepth][kPoolThreads];
+    __shared__ Entry s_stack[kWideDepth][kRayThreads<kEach>];
     const uint32_t root = __ldg(rootPtr);
     const bool unusable = kQuant && __ldg(status) != 0u;
     f3 ro = mk(0, 0, 0), rd = ro, inv = ro;
@@ -204,7 +212,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps<kAny> * 32 / kPoolThr
     int depth = 0;
     constexpr bool kReplayBinary = kQuant && !kAny && !kCount;
     bool binary = false;  // this ray walks the binary tree
-    trace_pool<kNodeSteps>(
+    trace_rays<kEach, kNodeSteps, kAny || kQuant ? 1 : kFewRounds>(
         rays, hits, pool, hit, curr,
         [&](uint32_t, float4 a, float4 b) {
             ro = mk(a.x, a.y, a.z);
@@ -230,13 +238,13 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolWarps<kAny> * 32 / kPoolThr
         [&] {
             if (kReplayBinary && binary)
                 return stackfree_replay_step<kAny, kCount, kReplayDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                                         kPoolThreads, hit, nodes, tris, ro, rd, inv,
+                                                                         kRayThreads<kEach>, hit, nodes, tris, ro, rd, inv,
                                                                          tmin, nv, nt);
             if constexpr (kAny)
-                return wide_any_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kPoolThreads, hit,
+                return wide_any_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kRayThreads<kEach>, hit,
                                                      slots, nodes, tris, leafTris, root, ro, rd, inv, tmin, nv, nt, nr);
             else
-                return wide_closest_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kPoolThreads,
+                return wide_closest_step<kCount, kQuant>(curr, prev, depth, &s_stack[0][threadIdx.x], kRayThreads<kEach>,
                                                          hit, slots, nodes, tris, leafTris, root, ro, rd, inv, tmin,
                                                          nv, nt, nr);
         },
@@ -291,18 +299,19 @@ mlbvh_status launch_trace_wide(const Slot* dSlots, const uint32_t* dStatus, cons
     const float* tris = reinterpret_cast<const float*>(dTris);
     const bool any = rayQuery == MLBVH_RAY_QUERY_ANY;
     const RayPool pool = ray_pool(nRays, device_sm_count(), any ? kPoolWarps<true> : kPoolWarps<false>);
-    if (any && dCounts)
-        k_trace_wide<true, true, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, dCounts, pool);
-    else if (any)
-        k_trace_wide<true, false, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nullptr, pool);
-    else if (dCounts)
-        k_trace_wide<false, true, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, dCounts, pool);
+    auto launch = [&](auto each) {
+        constexpr bool kEach = decltype(each)::value;
+        const auto kernel = any ? (dCounts ? k_trace_wide<true, true, kQuant, kEach, Slot>
+                                           : k_trace_wide<true, false, kQuant, kEach, Slot>)
+                                : (dCounts ? k_trace_wide<false, true, kQuant, kEach, Slot>
+                                           : k_trace_wide<false, false, kQuant, kEach, Slot>);
+        kernel<<<ray_ctas(pool, kEach), kRayThreads<kEach>, 0, stream>>>(dSlots, dStatus, dNodes, dRoot, tris, dLeafTris,
+                                                                        rays, hits, dCounts, pool);
+    };
+    if ((any ? kEachRange<true> : kEachRange<false>).has(nRays, device_sm_count()))
+        launch(std::true_type{});
     else
-        k_trace_wide<false, false, kQuant><<<pool.ctas, kPoolThreads, 0, stream>>>(
-            dSlots, dStatus, dNodes, dRoot, tris, dLeafTris, rays, hits, nullptr, pool);
+        launch(std::false_type{});
     MLBVH_CHECK_LAUNCH("k_trace_wide");
     return MLBVH_OK;
 }
