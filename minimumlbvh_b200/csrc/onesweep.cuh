@@ -181,6 +181,17 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
     const Segment seg = s_seg;
     const uint32_t chunk = tile - seg.firstTile;
 
+    // on their way before the scan below, whose barriers the loads may not pass
+    const uint32_t localBase = chunk * (uint32_t)kTile + (uint32_t)warp * (kPer * 32);
+    uint32_t key[kPer], val[kPer], rank[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const uint32_t li = localBase + k * 32 + lane;
+        const bool valid = li < seg.len;
+        key[k] = valid ? chain_load(keysIn + seg.start + li) : 0xFFFFFFFFu;
+        val[k] = kFirst ? li : (valid ? chain_load(valsIn + seg.start + li) : 0u);
+    }
+
     // global start of every digit of this thread (digit d = j * kThreads + tid)
     uint32_t digitBase[kDPT], count[kDPT];
     {
@@ -194,15 +205,6 @@ __global__ void __launch_bounds__(kThreads, kBits == 8 ? 3 : 1)
         }
     }
 
-    const uint32_t localBase = chunk * (uint32_t)kTile + (uint32_t)warp * (kPer * 32);
-    uint32_t key[kPer], val[kPer], rank[kPer];
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        const uint32_t li = localBase + k * 32 + lane;
-        const bool valid = li < seg.len;
-        key[k] = valid ? chain_load(keysIn + seg.start + li) : 0xFFFFFFFFu;
-        val[k] = kFirst ? li : (valid ? chain_load(valsIn + seg.start + li) : 0u);
-    }
     const uint32_t lanesBelow = (1u << lane) - 1u;
     uint32_t* myHist = s_warpHist + warp * kBins;
 #pragma unroll
