@@ -20,14 +20,14 @@
 //                     histograms per mesh, reset of the hand-off words
 //   k_onesweep x P    segmented Onesweep passes (onesweep.cuh), one segment
 //                     per mesh; P = 4 (8-bit digits) or 3 (11-bit digits)
-//   k_tree_tiles, k_tree_cross   the trees, as mlbvh_build (tree.cuh)
+//   k_tree_tiles, k_tree_groups, k_tree_cross   the trees, as mlbvh_build (tree.cuh)
 //
 // Traversal: k_batch_trace is persistent (one grid of resident CTAs). A warp
 // takes `queueChunk` consecutive rays per atomic on the queue counter and
-// hands them to its idle lanes; every lane walks its own ray one node per
-// loop iteration (the stack-free walk of intersect_stackfree, or the replay
-// walk that gives the same Hit records from a stack of pending far children)
-// and takes the next ray as soon as it finishes, so lanes never wait for the
+// hands them to its idle lanes; every lane walks its own ray, up to 5 node
+// visits and one leaf test per loop iteration (the stack-free walk of
+// intersect_stackfree, or the replay walk that gives the same Hit records from
+// a stack of pending far children), and takes the next ray as soon as it finishes, so lanes never wait for the
 // longest ray of the warp. Rays find their mesh through the ray offsets.
 #include <algorithm>
 #include <cstring>

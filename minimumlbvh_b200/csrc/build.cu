@@ -14,7 +14,7 @@
 //   k_onesweep x4    one stable pass per digit: warp multisplit, decoupled
 //                    look-back over per-tile digit counts, scatter through
 //                    shared memory so that runs of one digit store coalesced
-//   k_tree_tiles, k_tree_cross   the tree (build_lbvh, minimum_lbvh.h:284-361;
+//   k_tree_tiles, k_tree_groups, k_tree_cross   the tree (build_lbvh, minimum_lbvh.h:284-361;
 //                    tree.cuh)
 #include <algorithm>
 #include <cstdio>
