@@ -421,7 +421,8 @@ mlbvh_status pt_diff_render(float* dImage, int w, int h, int spp, int bounces, c
     if (mlbvh_status s = check_diff_args(w, h, spp, bounces, dImage, dRoot, dTris, dAlbedo, dEmission)) return s;
     if (!aligned32(dNodes)) return fail(MLBVH_ERR_INVALID_ARG, "device pointers must be 16-byte aligned");
     if ((long long)w * h * 32 >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
-    DiffScene sc{w, h, spp, bounces, 0, 0, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo, dEmission};
+    DiffScene sc{w, h, spp, bounces, 0, 0, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo,
+                 dEmission};
     if (pixel_warps(sc)) {
         k_pt_diff_render_pixel<<<(unsigned)(w * h), 32, 0, stream>>>(dImage, sc);
     } else {
@@ -441,7 +442,8 @@ mlbvh_status pt_diff_adjoint(float* dGrad, const float* dGradImage, int w, int h
     if (!dGradImage || !aligned16(dGradImage) || !aligned32(dNodes))
         return fail(MLBVH_ERR_INVALID_ARG, "null or misaligned pointer");
     if ((long long)w * h * 32 >= (1ll << 31)) return fail(MLBVH_ERR_INVALID_ARG, "bad image size");
-    DiffScene sc{w, h, spp, bounces, 0, 0, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo, dEmission};
+    DiffScene sc{w, h, spp, bounces, 0, 0, cam, dRoot, dNodes, reinterpret_cast<const float*>(dTris), dAlbedo,
+                 dEmission};
     if (pixel_warps(sc)) {
         k_pt_diff_adjoint_pixel<<<(unsigned)(w * h), 32, 0, stream>>>(dGrad, dGradImage, sc);
     } else {

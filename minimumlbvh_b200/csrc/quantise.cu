@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kQuantiseThreads)
 // counts (may be null): per ray, internal-node visits, triangle tests and
 // parent loads at counts[i], counts[pool.n + i], counts[2n + i].
 template <bool kAny, int kDepth, bool kCount, bool kEach>
-__global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps<kAny> : kPoolWarps) * 32 / kRayThreads<kEach>)
+__global__ void __launch_bounds__(kRayThreads<kEach>,
+                                  (kEach ? kEachWarps<kAny> : kPoolWarps) * 32 / kRayThreads<kEach>)
     k_trace_quantised(const mlbvh_qnode* __restrict__ qnodes, const uint32_t* __restrict__ parents,
                       const mlbvh_qtri* __restrict__ qtris, const mlbvh_qheader* __restrict__ header,
                       const float4* __restrict__ rays, float4* __restrict__ hits,
@@ -246,8 +247,8 @@ __global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps<kAny> 
                                                     nt, nu);
             else
                 return quantised_replay_step<kAny, kCount, kDepth>(curr, prev, depth, &s_stack[0][threadIdx.x],
-                                                                   kRayThreads<kEach>, hit, qnodes, parents, qtris, qp, ro,
-                                                                   rd, inv, tmin, nv, nt, nu);
+                                                                   kRayThreads<kEach>, hit, qnodes, parents, qtris, qp,
+                                                                   ro, rd, inv, tmin, nv, nt, nu);
         },
         [&](uint32_t i) {
             if (kCount) {
@@ -265,9 +266,11 @@ void launch_trace_quantised(cudaStream_t stream, const mlbvh_qnode* q, const uin
 {
     const RayPool pool = ray_pool(n, device_sm_count(), kPoolWarps);
     const bool each = kEachRange<kAny>.has(n, device_sm_count());
-    const auto kernel = counts ? (each ? k_trace_quantised<kAny, kDepth, true, true> : k_trace_quantised<kAny, kDepth, true, false>)
-                               : (each ? k_trace_quantised<kAny, kDepth, false, true> : k_trace_quantised<kAny, kDepth, false, false>);
-    kernel<<<ray_ctas(pool, each), each ? kEachThreads : kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, counts, pool);
+    const auto kernel =
+        counts ? (each ? k_trace_quantised<kAny, kDepth, true, true> : k_trace_quantised<kAny, kDepth, true, false>)
+               : (each ? k_trace_quantised<kAny, kDepth, false, true> : k_trace_quantised<kAny, kDepth, false, false>);
+    kernel<<<ray_ctas(pool, each), each ? kEachThreads : kPoolThreads, 0, stream>>>(q, p, t, h, rays, hits, counts,
+                                                                                    pool);
 }
 
 template <bool kAny>

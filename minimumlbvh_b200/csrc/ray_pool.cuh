@@ -25,8 +25,9 @@ constexpr uint32_t kFewLanes = 16;   // below, a warp's round is kFew rounds of 
 
 // The pool of a query of n rays: one CTA per block of 32 rays (fewer rays where
 // that leaves multiprocessors idle), as many CTAs as are resident at most; block
-// b goes to CTA b modulo their number, so that neighbouring rays, which cost alike, are spread over all CTAs. Where the CTA
-// has fewer rays than lanes, its warps share them out.
+// b goes to CTA b modulo their number, so that neighbouring rays, which cost
+// alike, are spread over all CTAs. Where the CTA has fewer rays than lanes, its
+// warps share them out.
 struct RayPool {
     uint32_t n, ctas, lanes, shift;  // rays, CTAs, lanes used of each warp, log2 of the block
 };

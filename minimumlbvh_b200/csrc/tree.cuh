@@ -326,7 +326,9 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupCtas)
         last = atomicAdd(sc.counts + (g >> 5), 1u) == min(32u, groups - (g & ~31u)) - 1;
         __threadfence();
     }
-    if (__shfl_sync(0xffffffffu, last, 0)) reduce_block(sc.level[1], sc.level[2], groups, g >> 5);
+    last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();  // the first lane's fence holds for all
+    if (last) reduce_block(sc.level[1], sc.level[2], groups, g >> 5);
 }
 
 // The next tile's inputs of one thread: its leaf's triangle (copied to shared

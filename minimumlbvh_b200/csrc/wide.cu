@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(kWideThreads)
 // to the stack-free walk, or for closest hits without counters to the replay
 // walk, which returns the same Hit records.
 template <bool kAny, bool kCount, bool kQuant, bool kEach, class Slot>
-__global__ void __launch_bounds__(kRayThreads<kEach>, (kEach ? kEachWarps<kAny> : kPoolWarps<kAny>) * 32 / kRayThreads<kEach>)
+__global__ void __launch_bounds__(kRayThreads<kEach>,
+                                  (kEach ? kEachWarps<kAny> : kPoolWarps<kAny>) * 32 / kRayThreads<kEach>)
     k_trace_wide(const Slot* __restrict__ slots, const uint32_t* __restrict__ status,
                  const mlbvh_internal_node* __restrict__ nodes, const mlbvh_node_index* __restrict__ rootPtr,
                  const float* __restrict__ tris, const mlbvh_qtri* __restrict__ leafTris,
@@ -308,7 +309,7 @@ mlbvh_status launch_trace_wide(const Slot* dSlots, const uint32_t* dStatus, cons
         kernel<<<ray_ctas(pool, kEach), kRayThreads<kEach>, 0, stream>>>(dSlots, dStatus, dNodes, dRoot, tris, dLeafTris,
                                                                         rays, hits, dCounts, pool);
     };
-    if ((any ? kEachRange<true> : kEachRange<false>).has(nRays, device_sm_count()))
+    if ((any ? kEachRange<true> : kEachRange<false>).has(nRays, device_sm_count()))  // see ray_pool.cuh
         launch(std::true_type{});
     else
         launch(std::false_type{});
