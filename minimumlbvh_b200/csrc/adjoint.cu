@@ -41,7 +41,7 @@ constexpr int kMaxBounces = 8;
 constexpr int kDiffStack = 16;       // replay-walk stack entries per lane (shared memory)
 constexpr uint32_t kUnit = 64;       // samples per unit of the render's ordered sums; two units are open at a time
 constexpr uint32_t kWarpSamples = 512;  // samples a warp takes where the image has enough pixels
-constexpr uint32_t kWidePixels = 30000;  // largest image that is shared out by single pixels
+constexpr uint32_t kWidePixels = 20000;  // largest image that is shared out by single pixels
 
 struct PathVertex {
     uint32_t tri;
@@ -59,7 +59,7 @@ __device__ __forceinline__ Camera camera_of(const mlbvh_ray_generator& g)
 
 struct DiffScene {
     int w, h, spp, bounces;
-    uint32_t warps, shift;  // warps that share the pixels out in groups of 1 << shift
+    uint32_t warps, group;  // warps that share the pixels out in groups of so many
     mlbvh_ray_generator gen;
     const mlbvh_node_index* rootPtr;
     const mlbvh_internal_node* nodes;
@@ -111,14 +111,15 @@ __device__ __forceinline__ void trace_pixels(const DiffScene& sc, float* __restr
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t pixels = (uint32_t)(sc.w * sc.h), spp = (uint32_t)sc.spp;
     // the warp's pixels: group w, w + warps, ... of the image's; only the image's last group may be partial
-    const uint32_t group = 1u << sc.shift, groups = (pixels + group - 1) >> sc.shift;
+    const uint32_t groups = (pixels + sc.group - 1) / sc.group;
     const uint32_t w = blockIdx.x * (kDiffThreads / 32) + warp;
     if (w >= sc.warps) return;
-    uint32_t mine = ((groups - w + sc.warps - 1) / sc.warps) << sc.shift;
-    if ((groups - 1 - w) % sc.warps == 0) mine -= (groups << sc.shift) - pixels;
+    uint32_t mine = (groups - w + sc.warps - 1) / sc.warps * sc.group;
+    if ((groups - 1 - w) % sc.warps == 0) mine -= groups * sc.group - pixels;
     const uint32_t total = mine * spp;
     auto pixel_of = [&](uint32_t i) {  // the warp's i-th
-        return (((i >> sc.shift) * sc.warps + w) << sc.shift) + (i & (group - 1));
+        const uint32_t k = i / sc.group;
+        return (k * sc.warps + w - k) * sc.group + i;
     };
     const Camera cam = camera_of(sc.gen);
     const uint32_t root = __ldg(sc.rootPtr);
@@ -359,43 +360,52 @@ __global__ void __launch_bounds__(kDiffThreads, kDiffWarps * 32 / kDiffThreads)
     trace_pixels<true>(sc, nullptr, grad, gradImage);
 }
 
+// Views 2.5 times as wide as high and more: their long paths lie in a few
+// columns, the others end at once.
+bool is_wide(const DiffScene& sc) { return 2ll * sc.w >= 5ll * sc.h; }
+
 // The warps and their groups of pixels. A warp takes kWarpSamples samples at
 // most, four rounds of resident warps where that leaves it 128 samples, else two;
 // below 32, 32 samples (a warp's lanes share its instructions) as long as 16 warps
 // per SM remain: few samples finish soonest spread out. A group is as many pixels
-// as 32 samples need, so that the lanes trace neighbouring rays; single pixels in
-// small images at least four times as wide as high, whose paths are long in a few
-// columns only (400x60 and the like, 4 samples: 10 to 30 % faster). A warp's
-// samples stay below 2^31. Render and adjoint, 3 bounces, 213,000-triangle
+// as 32 samples need, so that the lanes trace neighbouring rays, or all of the
+// warp's where it has less than two such groups; a single pixel where its samples
+// nearly fill the warp, or half of it in a wide view, and in small wide views. A
+// warp's samples stay below 2^31. Render and adjoint, 3 bounces, 213,000-triangle
 // heightfield, us, with consecutive pixels in a warp / with groups all over the
 // image: 512x32, 32 samples 830 / 550; 400x60, 64 2,308 / 1,303; 1024x128, 32 4,987 /
-// 2,260; 512x512, 64 35,500 / 34,100, 4 2,969 / 2,925.
+// 2,260; 512x512, 64 35,500 / 34,100, 4 2,969 / 2,925. 180 images drawn over 32 to 512
+// pixels a side, 1 to 64 samples, 1 to 3 bounces: 1.08x on average, 0.945x to 1.6x.
 void share_out(DiffScene& sc)
 {
-    const unsigned long long pixels = (unsigned long long)sc.w * sc.h, samples = pixels * (unsigned long long)sc.spp;
-    const uint32_t sms = (uint32_t)device_sm_count(), spp = (uint32_t)sc.spp;
-    const unsigned long long round = samples / (kDiffWarps * sms);
-    unsigned long long k = std::min<unsigned long long>(std::max(round / 4, std::min(round / 2, 128ull)), kWarpSamples);
+    using u64 = unsigned long long;
+    const u64 w = (u64)sc.w, pixels = w * sc.h, spp = (u64)sc.spp, samples = pixels * spp;
+    const uint32_t sms = (uint32_t)device_sm_count();
+    const u64 round = samples / (kDiffWarps * sms);
+    u64 k = std::min<u64>(std::max(round / 4, std::min<u64>(round / 2, 128)), kWarpSamples);
     const bool few = k < 32;
-    if (few) k = std::max<unsigned long long>(1, std::min<unsigned long long>(32, samples / (16u * sms)));
-    if (!(few && pixels <= kWidePixels && sc.w / 4 >= sc.h))
-        while ((2ull << sc.shift) * spp <= std::min<unsigned long long>(k, 32)) ++sc.shift;
-    const unsigned long long groups = (pixels + (1u << sc.shift) - 1) >> sc.shift;
-    const unsigned long long per = std::max<unsigned long long>(1, k / ((1ull << sc.shift) * spp));
-    unsigned long long warps = (groups + per - 1) / per;
-    if (per > 1) {  // a warp's next group lies 0.38 of a row further on: never in the same columns
-        const unsigned long long w = (unsigned long long)sc.w, at = (warps << sc.shift) % w;
-        warps += ((w * 382 / 1000 + w - at) % w) >> sc.shift;
-    }
+    if (few) k = std::max<u64>(1, std::min<u64>(32, samples / (16u * sms)));
+    const bool single = spp >= (is_wide(sc) ? 16 : 24) || (few && is_wide(sc) && pixels <= kWidePixels);
+    const u64 lanes = k < 64 ? k : 32;  // samples of a group
+    const u64 group = single ? 1 : (lanes + spp - 1) / spp, groups = (pixels + group - 1) / group;
+    const u64 per = std::max<u64>(1, k / (group * spp));  // groups of a warp
+    u64 warps = (groups + per - 1) / per;
+    // a warp's next group lies 0.38 of a row further on: never in the same columns
+    if (per > 1) warps += (w * 382 / 1000 + w - warps * group % w) % w / group;
+    sc.group = (uint32_t)group;
     sc.warps = (uint32_t)std::min(warps, groups);
 }
-// A warp per pixel (trace_pixel). Render and adjoint, 3 bounces, against the
-// warps above, us: 32x32 at 1 / 4 / 8 / 16 samples 216 / 317 / 380 / 464 against 241 /
-// 340 / 386 / 472, 64x64 269 / 366 / 452 / 572 against 311 / 404 / 501 / 555; 80x80 314 /
-// 503 / 654 / 833 against 323 / 463 / 525 / 591.
+
+// A warp per pixel (trace_pixel): small images of few samples, wide ones up to
+// 16,000 pixels and 16 samples. Render and adjoint, 3 bounces, against the warps
+// above, us: 32x32 at 1 / 4 / 8 / 16 samples 216 / 317 / 380 / 464 against 241 / 340 / 386 /
+// 472, 64x64 269 / 366 / 452 / 572 against 311 / 404 / 501 / 555, 80x80 314 / 503 / 654 / 833
+// against 323 / 463 / 525 / 591; 300x40 at 4 samples 348 against 388.
 bool pixel_warps(const DiffScene& sc)
 {
-    return sc.spp <= 8 && (uint32_t)sc.w * (uint32_t)sc.h <= 32u * (uint32_t)device_sm_count();
+    const uint32_t pixels = (uint32_t)sc.w * (uint32_t)sc.h, spp = (uint32_t)sc.spp, sms = (uint32_t)device_sm_count();
+    if (is_wide(sc)) return spp <= 16 && pixels <= 108 * sms;
+    return spp <= 12 && pixels <= 52 * sms && pixels * spp <= 256 * sms;
 }
 uint32_t diff_blocks(const DiffScene& sc) { return (sc.warps + kDiffThreads / 32 - 1) / (kDiffThreads / 32); }
 

@@ -1,9 +1,11 @@
-"""How the differentiable kernels share an image out: a warp per pixel up to 32
-pixels per multiprocessor and 8 samples, else groups of pixels all over the
-image, single pixels in wide images of few samples; strides that would fall
-into the same columns, partial last groups. The image against the oracle's bit
-for bit, the gradient against its FP64 adjoint (1e-3 relative, as
-test_gpu_adjoint.py, at triangles with at least 1 % of the largest)."""
+"""How the differentiable kernels share an image out: a warp per pixel in small
+images of few samples (up to 52 pixels and 256 samples per multiprocessor, 108
+pixels and 16 samples in views at least 2.5 times as wide as high), else groups
+of pixels all over the image, single pixels of many samples or in wide views;
+strides that would fall into the same columns, partial last groups. The image
+against the oracle's bit for bit, the gradient against its FP64 adjoint (1e-3
+relative, as test_gpu_adjoint.py, at triangles with at least 1 % of the
+largest)."""
 import numpy as np
 import pytest
 
@@ -23,7 +25,9 @@ def scene(cuda):
 
 
 @pytest.mark.parametrize("w,h,spp", [(64, 74, 8), (64, 74, 9), (149, 32, 8), (1, 1, 3), (300, 40, 4), (401, 61, 2),
-                                     (400, 60, 64), (512, 32, 33), (201, 201, 5), (131, 97, 1)])
+                                     (400, 60, 64), (512, 32, 33), (201, 201, 5), (131, 97, 1), (104, 74, 4),
+                                     (105, 74, 4), (50, 63, 12), (50, 63, 13), (216, 74, 16), (217, 74, 16),
+                                     (216, 74, 17), (101, 67, 24), (101, 67, 23), (260, 113, 3)])
 def test_image_and_gradient(scene, w, h, spp):
     import torch
     tris, alb, em, b, t, out = scene
